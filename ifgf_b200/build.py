@@ -23,7 +23,8 @@ SOURCES = ["operator.cu", "plan.cpp", "gpu_tree.cu", "gpu_lists.cu", "gpu_target
     f"kernels_k{k}.cu" for k in range(8)]
 HEADERS = ["common.hpp", "devbuf.hpp", "gpu_target_lists.hpp", "plan.hpp", "operator.hpp",
            "device_math.cuh", "mult.hpp",
-           "mult_kernels.cuh", "mult_batch.cuh", "far_staged.cuh", "tcgen05.cuh", "upward_tc.cuh"]
+           "mult_kernels.cuh", "mult_batch.cuh", "far_staged.cuh", "tcgen05.cuh", "upward_tc.cuh",
+           "upward_staged64.cuh"]
 
 
 def _newer(target, deps):

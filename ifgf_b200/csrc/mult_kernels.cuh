@@ -1523,6 +1523,8 @@ __global__ void __launch_bounds__(UPS_THREADS, 8) upward_staged_kernel(UpArgs a)
         cv[(size_t)c * a.P_hi + n] = acc[n];
 }
 
+#include "upward_staged64.cuh"
+
 } // namespace ifgf
 #include "upward_tc.cuh"
 namespace ifgf
@@ -2303,6 +2305,20 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
                                                             m.up_path, st, 1,
                                                             m.up_choice ? m.up_choice[l] : -1);
             }
+            if constexpr (!MIXED && N0 > 0)
+            {
+                ua.rch = ups64_rch<N0, N1, N2>(LL.fe_pad);
+                const size_t sm = ups64_smem<N0, N1, N2>(m.P_hi, ua.rch, LL.fe_pad);
+                if (LL.fe_pad > 0 && sm <= UP_STAGED_SMEM_MAX)
+                {
+                    auto kern = upward_staged64_kernel<KIND, N0, N1, N2>;
+                    if (sm > 48 * 1024)
+                        IFGF_CHECK(cudaFuncSetAttribute(
+                            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                    kern<<<LL.n_up, UPS64_THREADS, sm, st>>>(ua);
+                    staged = true;
+                }
+            }
             if constexpr (MIXED && N0 > 0 && (N0 * N1 * N2) % 2 == 0)
                 if (!staged)
             {
@@ -2325,7 +2341,7 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
                 upward_mixed_kernel<KIND, N0, N1, N2>
                     <<<LL.n_up, UP_THREADS, m.P_hi * sizeof(float2), st>>>(ua);
             else
-                upward_kernel<KIND, N0, N1, N2>
+                upward_kernel<KIND, 0, 0, 0>
                     <<<LL.n_up, UP_THREADS, m.P_hi * sizeof(double2), st>>>(ua);
             IFGF_CHECK_LAUNCH();
             if (hk)
