@@ -2,6 +2,8 @@
 // coordinates, cone lookups, Chebyshev evaluation and the six kernel plug-ins.
 #pragma once
 
+#include <cmath>
+
 #include <cuda_runtime.h>
 
 #include "common.hpp"
@@ -40,11 +42,22 @@ constexpr double DPI = 3.14159265358979323846;
 // Wavenumber and plug-in switches shared by all kernels of one operator.
 struct KParams
 {
+    static constexpr bool NORMAL = false; // squared distances may be zero or subnormal
     double kr, ki; // k = kr + i ki (real kernels use kr)
     int dx;        // GradHelmholtz derivative direction, -1 = plain single layer
     // kr and ki split into two floats each (hi + lo), for the mixed pipeline
     float krh, krl, kih, kil;
+    // FP64 phases and damping in the units their reductions use, as hi + lo
+    // pairs: quarter turns 2 kr / pi and -2 ki / pi, octaves -kr / ln 2
+    double qrh, qrl, qih, qil, erh, erl;
 };
+
+// a (bh + bl) as an unevaluated sum
+inline void scaled_pair(double a, double bh, double bl, double* h, double* l)
+{
+    *h = a * bh;
+    *l = fma(a, bh, -*h) + a * bl;
+}
 
 inline KParams make_kparams(double kr, double ki, int dx)
 {
@@ -56,23 +69,179 @@ inline KParams make_kparams(double kr, double ki, int dx)
     p.krl = (float)(kr - (double)p.krh);
     p.kih = (float)ki;
     p.kil = (float)(ki - (double)p.kih);
+    // 2 / pi and 1 / ln 2 as hi + lo pairs
+    constexpr double TWO_PI_H = 0.6366197723675814, TWO_PI_L = -3.935735335036497e-17;
+    constexpr double LOG2E_H = 1.4426950408889634, LOG2E_L = 2.0355273740931033e-17;
+    scaled_pair(kr, TWO_PI_H, TWO_PI_L, &p.qrh, &p.qrl);
+    scaled_pair(-ki, TWO_PI_H, TWO_PI_L, &p.qih, &p.qil);
+    scaled_pair(-kr, LOG2E_H, LOG2E_L, &p.erh, &p.erl);
     return p;
 }
 
-// e^{-k d} for complex k: e^{-kr d} (cos(ki d), -sin(ki d))
-__device__ __forceinline__ cplx<double> exp_mk(const KParams& p, double d)
+// ---------------------------------------------------------------------------
+// FP64 distance, phase and damping of the kernels.  With the library's square
+// root, division and sincos a Helmholtz (source, node) pair took about 150
+// instructions, 55 of them on the FP64 pipe; the forms below take about 75
+// and 42 and are at least as accurate (the phase k d is never rounded: its
+// reduction is exact through FMA; sums of 400 terms at k d <= 200 against
+// extended precision: 4.1e-15 relative, 4.9e-15 with the library's).
+// ---------------------------------------------------------------------------
+struct DistInv
 {
-    double s, c;
-    sincos(-p.ki * d, &s, &c);
-    const double m = exp(-p.kr * d);
-    return {m * c, m * s};
+    double d, id; // sqrt(d2), 1 / sqrt(d2)
+};
+
+// whether d2 >= 0 is zero or subnormal
+__device__ __forceinline__ bool tiny_square(double d2)
+{
+    return (unsigned)__double2hiint(d2) < 0x00100000u;
+}
+
+// The hardware's reciprocal-square-root estimate (about 20 bits), one step of
+// Halley's third-order iteration y (1 + e / 2 + 3 e^2 / 8), e = 1 - x y^2
+// (residual 5 e^3 / 16, below 2^-54), and one Newton correction of the root.
+// Unless NORMAL (the caller has seen that d2 is a normal number), zero and
+// subnormal squares are scaled first; d2 = 0 gives d = 0, id = inf.
+template <bool NORMAL> __device__ __forceinline__ DistInv dist_inv(double d2)
+{
+    const bool tiny = !NORMAL && tiny_square(d2);
+    double x = d2, y;
+    if (tiny)
+        x = d2 * 0x1p200;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    DistInv q;
+    q.id = fma(fma(0.375, e, 0.5), e * y, y);
+    const double d0 = x * q.id;
+    // half the estimate (its exponent less one) is accurate enough here
+    const double h = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));
+    q.d = fma(fma(-d0, d0, x), h, d0);
+    if (tiny)
+    {
+        q.d = d2 == 0.0 ? 0.0 : q.d * 0x1p-100;
+        q.id = d2 == 0.0 ? __longlong_as_double(0x7ff0000000000000ll) : q.id * 0x1p100;
+    }
+    return q;
+}
+// Polynomials through Chebyshev points (exact rational arithmetic, rounded):
+// sin(pi r / 2) / r in r^2 (the constant term as a hi + lo pair) and
+// (cos(pi r / 2) - 1) / r^2 in r^2 for |r| <= 1/2 (truncation 4e-18 and 1e-19
+// of the result), (2^f - 1) / f for |f| <= 1/2 (1e-17 of 2^f).
+constexpr int TRIG_N = 15, EXP2_N = 11;
+#define IFGF_TRIG_C                                                                           \
+    1.5707963267948966, 5.628876619455937e-17, -0.6459640975062443, 0.07969262624604301,       \
+        -0.004681754132340976, 0.0001604411507421909, -3.598643352982311e-06,                  \
+        5.633933781538053e-08, -1.2337005501361697, 0.2536695079010478, -0.020863480763340773, \
+        0.0009192602745468447, -2.5202039028029178e-05, 4.7106784055052287e-07,                \
+        -6.329396344967619e-09
+#define IFGF_EXP2_C                                                                           \
+    0.6931471805599453, 0.24022650695910097, 0.0555041086648216, 0.009618129107606888,         \
+        0.0013333558146416936, 0.0001540353044173605, 1.525273382983612e-05,                   \
+        1.321544258792169e-06, 1.0178062445845774e-07, 7.072585949269187e-09,                  \
+        4.454960598186499e-10
+struct PolyConst // the coefficients as compile-time constants
+{
+    __device__ static constexpr double trig(int i)
+    {
+        constexpr double c[TRIG_N] = {IFGF_TRIG_C};
+        return c[i];
+    }
+    __device__ static constexpr double exp2(int i)
+    {
+        constexpr double c[EXP2_N] = {IFGF_EXP2_C};
+        return c[i];
+    }
+};
+// The same values in memory, for loops that keep them in registers: as
+// constants every use in a loop loads its coefficient again (111 instead of
+// 78 instructions per leaf evaluation).
+static __device__ double poly_mem[TRIG_N + EXP2_N] = {IFGF_TRIG_C, IFGF_EXP2_C};
+struct PolyRegs
+{
+    double t[TRIG_N], e[EXP2_N];
+    __device__ __forceinline__ PolyRegs()
+    {
+#pragma unroll
+        for (int i = 0; i < TRIG_N; i++)
+            t[i] = poly_mem[i];
+#pragma unroll
+        for (int i = 0; i < EXP2_N; i++)
+            e[i] = poly_mem[TRIG_N + i];
+    }
+    __device__ __forceinline__ double trig(int i) const { return t[i]; }
+    __device__ __forceinline__ double exp2(int i) const { return e[i]; }
+};
+// KParams of a loop that keeps the coefficients in registers and has seen
+// that the squared distances are normal numbers
+struct KParamsRegs : KParams
+{
+    static constexpr bool NORMAL = true;
+    PolyRegs c;
+    __device__ __forceinline__ explicit KParamsRegs(const KParams& p) : KParams(p) {}
+};
+__device__ __forceinline__ PolyConst poly_of(const KParams&) { return {}; }
+__device__ __forceinline__ const PolyRegs& poly_of(const KParamsRegs& p) { return p.c; }
+
+// adding 1.5 2^52 rounds to an integer, held in the sum's low bits
+constexpr double ROUND_MAGIC = 6755399441055744.0;
+
+// e^{i (pi / 2) (qh + ql) d}: the quarter turns q d less their nearest integer
+// are formed exactly by FMA, |r| <= 1/2
+template <class C>
+__device__ __forceinline__ cplx<double> quarter_turns(double qh, double ql, double d, const C& k)
+{
+    const double m = fma(qh, d, ROUND_MAGIC);
+    const int n = __double2loint(m);
+    double r = fma(qh, d, -(m - ROUND_MAGIC));
+    r = fma(ql, d, r);
+    const double z = r * r;
+    double sp = k.trig(7), cp = k.trig(14);
+#pragma unroll
+    for (int i = 6; i >= 1; i--)
+        sp = fma(sp, z, k.trig(i));
+#pragma unroll
+    for (int i = 13; i >= 8; i--)
+        cp = fma(cp, z, k.trig(i));
+    const double s = fma(r, k.trig(0), r * sp);
+    const double c = fma(cp, z, 1.0);
+    // quarter n mod 4: swap for odd n, negate the cosine for 1 and 2, the
+    // sine for 2 and 3
+    const bool odd = n & 1;
+    const double cc = odd ? s : c, ss = odd ? c : s;
+    return {__hiloint2double(__double2hiint(cc) ^ (((n + 1) & 2) << 30), __double2loint(cc)),
+            __hiloint2double(__double2hiint(ss) ^ ((n & 2) << 30), __double2loint(ss))};
+}
+
+// e^{-kr d} as 2^t, t = (erh + erl) d: 2^f scaled through the exponent field.
+// Without branches (they would keep the compiler from interleaving a
+// thread's evaluations): beyond the normal range the result is infinity, or
+// zero (from 2^-1021 down).
+template <class KP> __device__ __forceinline__ double damping(const KP& p, double d)
+{
+    const double m = fma(p.erh, d, ROUND_MAGIC);
+    const int n = __double2loint(m), mh = __double2hiint(m);
+    const double f = fma(p.erl, d, fma(p.erh, d, -(m - ROUND_MAGIC)));
+    const auto& k = poly_of(p);
+    double e = k.exp2(EXP2_N - 1);
+#pragma unroll
+    for (int i = EXP2_N - 2; i >= 0; i--)
+        e = fma(e, f, k.exp2(i));
+    e = fma(e, f, 1.0);
+    // m's high word is 0x43380000 (0x4337ffff) for 0 <= n (< 0) in 32 bits
+    const bool in = (unsigned)(n + 1021) <= 2044u && (unsigned)(mh - 0x4337ffff) <= 1u;
+    const int hi = in ? __double2hiint(e) + (n << 20) : (mh < 0x43380000 ? 0 : 0x7ff00000);
+    return __hiloint2double(hi, in ? __double2loint(e) : 0);
+}
+
+// f e^{-k d} for complex k: f e^{-kr d} (cos(ki d), -sin(ki d))
+template <class KP> __device__ __forceinline__ cplx<double> exp_mk(const KP& p, double d, double f)
+{
+    return cscale(quarter_turns(p.qih, p.qil, d, poly_of(p)), f * damping(p, d));
 }
 // e^{i k d} for real k
-__device__ __forceinline__ cplx<double> exp_ik(double k, double d)
+template <class KP> __device__ __forceinline__ cplx<double> exp_ik(const KP& p, double d)
 {
-    double s, c;
-    sincos(k * d, &s, &c);
-    return {c, s};
+    return quarter_turns(p.qrh, p.qrl, d, poly_of(p));
 }
 
 // ---------------------------------------------------------------------------
@@ -225,33 +394,52 @@ __device__ __forceinline__ cplx<double> cheb_eval3(const double2* __restrict__ c
 // ---------------------------------------------------------------------------
 // Kernel plug-ins.  x = x_src - y_tgt throughout, as in the reference's
 // evaluateKernel loops (e.g. helmholtz_ifgf.hpp:104-111).
+//   kernel4pi  4 pi G
+//   cf         centred factor G(y, xc) (its modulus without the kernel's order)
+//   transfer   centre shift G(y, x_child) / G(y, x_parent)
+//   leaf_add   s += w G(y, x) / G(y, xc) / leaf_scale(dc) with a = x - y and
+//              dc = |y - xc|: the factor that depends on the node alone is
+//              applied once to the sum
+// kernel4pi and leaf_add take KParams, or KParamsRegs where the caller knows
+// that |x|^2 (|a|^2) is a normal number.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ double dot3(const double* a, const double* b)
+{
+    return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+}
+// component dx of a (a dynamic index would put a in local memory)
+__device__ __forceinline__ double component(const double* a, int dx)
+{
+    return dx == 0 ? a[0] : (dx == 1 ? a[1] : a[2]);
+}
+
 template <int KIND> struct Plugin;
 
 // laplace_ifgf.hpp
 template <> struct Plugin<K_LAPLACE>
 {
     static constexpr bool needs_normals = false;
-    __device__ static cplx<double> kernel(const double* x, const double*, const KParams&)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP&)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        return {(d == 0) ? 0.0 : INV4PI / d, 0.0};
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
+        return {!KP::NORMAL && q.d == 0 ? 0.0 : q.id, 0.0};
     }
     __device__ static cplx<double> cf(const double* x, const KParams&)
     {
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        return {(1.0 / sqrt(d2)) * INV4PI, 0.0};
+        return {dist_inv<false>(dot3(x, x)).id * INV4PI, 0.0};
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams&)
     {
         return {sqrt(dp2) / sqrt(d2), 0.0};
     }
-    // w * G(y, x)/G(y, xc) with a = x - y
-    __device__ static cplx<double> factored(const double* a, const double*, cplx<double> w,
-                                            const double*, double dc, const KParams&)
+    __device__ static double leaf_scale(double dc) { return dc; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double*,
+                                    cplx<double> w, double, const KP&)
     {
-        const double d = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-        return {(d == 0) ? 0.0 : w.re * dc / d, 0.0};
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(a, a));
+        s.re = fma(w.re, !KP::NORMAL && q.d == 0 ? 0.0 : q.id, s.re);
     }
 };
 
@@ -259,32 +447,29 @@ template <> struct Plugin<K_LAPLACE>
 template <> struct Plugin<K_HELMHOLTZ>
 {
     static constexpr bool needs_normals = false;
-    __device__ static cplx<double> kernel(const double* x, const double*, const KParams& p)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        if (d == 0)
-            return {0.0, 0.0};
-        const cplx<double> e = exp_ik(p.kr, d);
-        const double f = INV4PI / d;
-        return {e.re * f, e.im * f};
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
+        return cscale(exp_ik(p, q.d), !KP::NORMAL && q.d == 0 ? 0.0 : q.id);
     }
     __device__ static cplx<double> cf(const double* x, const KParams& p)
     {
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        const double id = 1.0 / sqrt(d2);
-        const double d = d2 * id;
-        return cscale(exp_ik(p.kr, d), id * INV4PI);
+        const DistInv q = dist_inv<false>(dot3(x, x));
+        return cscale(exp_ik(p, q.d), q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
         const double d = sqrt(d2), dp = sqrt(dp2);
-        return cscale(exp_ik(p.kr, d - dp), dp / d);
+        return cscale(exp_ik(p, d - dp), dp / d);
     }
-    __device__ static cplx<double> factored(const double* a, const double*, cplx<double> w,
-                                            const double*, double dc, const KParams& p)
+    __device__ static double leaf_scale(double dc) { return dc; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double*,
+                                    cplx<double> w, double dc, const KP& p)
     {
-        const double d = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-        return cmul(w, cscale(exp_ik(p.kr, d - dc), dc / d));
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(a, a));
+        cfma(s, w, cscale(exp_ik(p, q.d - dc), q.id));
     }
 };
 
@@ -292,31 +477,29 @@ template <> struct Plugin<K_HELMHOLTZ>
 template <> struct Plugin<K_MODHELMHOLTZ>
 {
     static constexpr bool needs_normals = false;
-    __device__ static cplx<double> kernel(const double* x, const double*, const KParams& p)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        if (d == 0)
-            return {0.0, 0.0};
-        return cscale(exp_mk(p, d), INV4PI / d);
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
+        return exp_mk(p, q.d, !KP::NORMAL && q.d == 0 ? 0.0 : q.id);
     }
     __device__ static cplx<double> cf(const double* x, const KParams& p)
     {
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        const double id = 1.0 / sqrt(d2);
-        return cscale(exp_mk(p, d2 * id), id * INV4PI);
+        const DistInv q = dist_inv<false>(dot3(x, x));
+        return exp_mk(p, q.d, q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
         const double d = sqrt(d2), dp = sqrt(dp2);
-        return cscale(exp_mk(p, d - dp), dp / d);
+        return exp_mk(p, d - dp, dp / d);
     }
-    __device__ static cplx<double> factored(const double* a, const double*, cplx<double> w,
-                                            const double*, double dc, const KParams& p)
+    __device__ static double leaf_scale(double dc) { return dc; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double*,
+                                    cplx<double> w, double dc, const KP& p)
     {
-        const double d = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-        if (d == 0)
-            return {0.0, 0.0};
-        return cmul(w, cscale(exp_mk(p, d - dc), dc / d));
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(a, a));
+        cfma(s, w, exp_mk(p, q.d - dc, !KP::NORMAL && q.d == 0 ? 0.0 : q.id));
     }
 };
 
@@ -324,42 +507,43 @@ template <> struct Plugin<K_MODHELMHOLTZ>
 template <> struct Plugin<K_GRADHELMHOLTZ>
 {
     static constexpr bool needs_normals = false;
-    __device__ static cplx<double> kernel(const double* x, const double*, const KParams& p)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        if (d < 1e-12)
-            return {0.0, 0.0};
-        const cplx<double> e = exp_mk(p, d);
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
+        const double id = q.d < 1e-12 ? 0.0 : q.id;
         if (p.dx < 0)
-            return cscale(e, INV4PI / d);
-        // -(1/4pi) (1/d^2) e^{-kd} (-k - 1/d) x[dx]
-        const cplx<double> m = {-p.kr - 1.0 / d, -p.ki};
-        return cscale(cmul(e, m), -INV4PI * (1.0 / (d * d)) * x[p.dx]);
+            return exp_mk(p, q.d, id);
+        // -(1/d^2) e^{-kd} (-k - 1/d) x[dx]
+        const double f = (id * id) * component(x, p.dx);
+        return cmul(exp_mk(p, q.d, f), cplx<double>{p.kr + id, p.ki});
     }
     __device__ static cplx<double> cf(const double* x, const KParams& p)
     {
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        const double id = 1.0 / sqrt(d2);
-        return cscale(exp_mk(p, d2 * id), id * INV4PI);
+        const DistInv q = dist_inv<false>(dot3(x, x));
+        return exp_mk(p, q.d, q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
         const double invd = d2 > 1e-12 ? 1.0 / sqrt(d2) : 0.0;
         const double dp = sqrt(dp2), d = d2 * invd;
-        return cscale(exp_mk(p, d - dp), dp * invd);
+        return exp_mk(p, d - dp, dp * invd);
     }
-    __device__ static cplx<double> factored(const double* a, const double*, cplx<double> w,
-                                            const double*, double dc, const KParams& p)
+    __device__ static double leaf_scale(double dc) { return dc; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double*,
+                                    cplx<double> w, double dc, const KP& p)
     {
-        const double d2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
-        const double id = d2 > 1e-12 ? 1.0 / sqrt(d2) : 0.0;
-        const double d = d2 * id;
-        const cplx<double> e = cmul(w, exp_mk(p, d - dc));
+        const double d2 = dot3(a, a);
+        const DistInv q = dist_inv<KP::NORMAL>(d2);
+        const double id = d2 > 1e-12 ? q.id : 0.0, d = d2 > 1e-12 ? q.d : 0.0;
         if (p.dx < 0)
-            return cscale(e, dc * id);
-        const double ww = -(1.0 / d2) * dc * a[p.dx];
-        const cplx<double> m = {-p.kr - id, -p.ki};
-        return cscale(cmul(e, m), ww);
+        {
+            cfma(s, w, exp_mk(p, d - dc, id));
+            return;
+        }
+        const double f = (q.id * q.id) * component(a, p.dx);
+        cfma(s, w, cmul(exp_mk(p, d - dc, f), cplx<double>{p.kr + id, p.ki}));
     }
 };
 
@@ -367,83 +551,75 @@ template <> struct Plugin<K_GRADHELMHOLTZ>
 template <> struct Plugin<K_DOUBLELAYER>
 {
     static constexpr bool needs_normals = true;
-    __device__ static cplx<double> kernel(const double* x, const double* n, const KParams& p)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double* n, const KP& p)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        if (d < 1e-12)
-            return {0.0, 0.0};
-        const double xn = x[0] * n[0] + x[1] * n[1] + x[2] * n[2];
-        const cplx<double> m = {-p.kr - 1.0 / d, -p.ki};
-        return cscale(cmul(exp_mk(p, d), m), -INV4PI * (1.0 / (d * d)) * xn);
+        const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
+        const double id = q.d < 1e-12 ? 0.0 : q.id;
+        const double f = (id * id) * dot3(x, n);
+        return cmul(exp_mk(p, q.d, f), cplx<double>{p.kr + id, p.ki});
     }
     __device__ static cplx<double> cf(const double* x, const KParams& p)
     {
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        const double id = 1.0 / sqrt(d2);
-        return cscale(exp_mk(p, d2 * id), id * INV4PI);
+        const DistInv q = dist_inv<false>(dot3(x, x));
+        return exp_mk(p, q.d, q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
         const double invd = 1.0 / sqrt(d2);
         const double dp = sqrt(dp2), d = d2 * invd;
-        return cscale(exp_mk(p, d - dp), dp * invd);
+        return exp_mk(p, d - dp, dp * invd);
     }
-    __device__ static cplx<double> factored(const double* a, const double* n, cplx<double> w,
-                                            const double*, double dc, const KParams& p)
+    __device__ static double leaf_scale(double dc) { return dc; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double* n,
+                                    cplx<double> w, double dc, const KP& p)
     {
-        const double d2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
-        const double id = d2 > 1e-12 ? 1.0 / sqrt(d2) : 0.0;
-        const double d = d2 * id;
-        const double ww = -(1.0 / d2) * dc * (a[0] * n[0] + a[1] * n[1] + a[2] * n[2]);
-        const cplx<double> m = {-p.kr - id, -p.ki};
-        return cscale(cmul(cmul(w, exp_mk(p, d - dc)), m), ww);
+        const double d2 = dot3(a, a);
+        const DistInv q = dist_inv<KP::NORMAL>(d2);
+        const double id = d2 > 1e-12 ? q.id : 0.0, d = d2 > 1e-12 ? q.d : 0.0;
+        const double f = (q.id * q.id) * dot3(a, n);
+        cfma(s, w, cmul(exp_mk(p, d - dc, f), cplx<double>{p.kr + id, p.ki}));
     }
 };
 
-// combined_field_helmholtz_ifgf.hpp (real kappa, source normals)
+// combined_field_helmholtz_ifgf.hpp (real kappa, source normals):
+// e^{i kap d} / d^3 (nxy - i kap (d nxy + d^2)), nxy = -n . x
 template <> struct Plugin<K_COMBINEDFIELD>
 {
     static constexpr bool needs_normals = true;
-    __device__ static cplx<double> kernel(const double* x, const double* n, const KParams& p)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double* n, const KP& p)
     {
-        const double kap = p.kr;
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        const double invd = d2 < 1e-14 ? 0.0 : 1.0 / sqrt(d2);
-        const double d = d2 * invd;
-        const double nxy = -(n[0] * x[0] + n[1] * x[1] + n[2] * x[2]);
-        double s, c;
-        sincos(kap * d, &s, &c);
-        const double f = INV4PI * invd * invd * invd;
-        return {f * (c * nxy + s * kap * (d * nxy + d2)), f * (-c * kap * (d * nxy + d2) + s * nxy)};
+        const double d2 = dot3(x, x);
+        const DistInv q = dist_inv<KP::NORMAL>(d2);
+        const double id = d2 < 1e-14 ? 0.0 : q.id, d = d2 < 1e-14 ? 0.0 : q.d;
+        const double nxy = -dot3(n, x);
+        return cmul(cscale(exp_ik(p, d), id * id * id),
+                    cplx<double>{nxy, -p.kr * fma(d, nxy, d2)});
     }
     __device__ static cplx<double> cf(const double* x, const KParams& p)
     {
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        const double id = 1.0 / sqrt(d2);
-        return cscale(exp_ik(p.kr, d2 * id), id * INV4PI);
+        const DistInv q = dist_inv<false>(dot3(x, x));
+        return cscale(exp_ik(p, q.d), q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
         const double invd = 1.0 / sqrt(d2);
         const double dp = sqrt(dp2), d = d2 * invd;
-        return cscale(exp_ik(p.kr, d - dp), dp * invd);
+        return cscale(exp_ik(p, d - dp), dp * invd);
     }
-    __device__ static cplx<double> factored(const double* a, const double* n, cplx<double> w,
-                                            const double*, double dc, const KParams& p)
+    __device__ static double leaf_scale(double dc) { return dc; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double* n,
+                                    cplx<double> w, double dc, const KP& p)
     {
-        // z = y - x = -a
-        const double d2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
-        if (!(d2 > 1e-14))
-            return {0.0, 0.0};
-        const double kap = p.kr;
-        const double nxy = -(a[0] * n[0] + a[1] * n[1] + a[2] * n[2]);
-        const double id = 1.0 / sqrt(d2);
-        const double d = d2 * id;
-        double s, c;
-        sincos(kap * (d - dc), &s, &c);
-        const double f = dc / (d2 * d);
-        const double A = w.re * c - w.im * s, B = w.re * s + w.im * c;
-        return {f * (A * nxy + B * kap * (d * nxy + d2)), f * (-A * kap * (d * nxy + d2) + B * nxy)};
+        const double d2 = dot3(a, a);
+        const DistInv q = dist_inv<KP::NORMAL>(d2);
+        const double id = d2 > 1e-14 ? q.id : 0.0;
+        const double nxy = -dot3(a, n);
+        cfma(s, w, cmul(cscale(exp_ik(p, q.d - dc), id * id * id),
+                        cplx<double>{nxy, -p.kr * fma(q.d, nxy, d2)}));
     }
 };
 
@@ -454,29 +630,29 @@ template <> struct Plugin<K_COMBINEDFIELD>
 template <> struct Plugin<K_HELMHOLTZ_DK>
 {
     static constexpr bool needs_normals = false;
-    __device__ static cplx<double> kernel(const double* x, const double*, const KParams& p)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        if (d == 0)
-            return {0.0, 0.0};
-        const cplx<double> e = exp_ik(p.kr, d);
-        return {-e.im * INV4PI, e.re * INV4PI};
+        const double d = dist_inv<KP::NORMAL>(dot3(x, x)).d;
+        const cplx<double> e = exp_ik(p, d);
+        const bool zero = !KP::NORMAL && d == 0;
+        return {zero ? 0.0 : -e.im, zero ? 0.0 : e.re};
     }
     __device__ static cplx<double> cf(const double* x, const KParams& p)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        return cscale(exp_ik(p.kr, d), INV4PI);
+        return cscale(exp_ik(p, dist_inv<false>(dot3(x, x)).d), INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
-        return exp_ik(p.kr, sqrt(d2) - sqrt(dp2));
+        return exp_ik(p, sqrt(d2) - sqrt(dp2));
     }
-    __device__ static cplx<double> factored(const double* a, const double*, cplx<double> w,
-                                            const double*, double dc, const KParams& p)
+    __device__ static double leaf_scale(double) { return 1.0; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double*,
+                                    cplx<double> w, double dc, const KP& p)
     {
-        const double d = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
-        const cplx<double> v = cmul(w, exp_ik(p.kr, d - dc));
-        return {-v.im, v.re};
+        const cplx<double> e = exp_ik(p, dist_inv<KP::NORMAL>(dot3(a, a)).d - dc);
+        cfma(s, w, cplx<double>{-e.im, e.re});
     }
 };
 
@@ -486,42 +662,32 @@ template <> struct Plugin<K_HELMHOLTZ_DK>
 template <> struct Plugin<K_COMBINEDFIELD_DK>
 {
     static constexpr bool needs_normals = true;
-    __device__ static cplx<double> kernel(const double* x, const double* n, const KParams& p)
+    template <class KP>
+    __device__ static cplx<double> kernel4pi(const double* x, const double* n, const KP& p)
     {
-        const double kap = p.kr;
-        const double d2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-        if (d2 < 1e-14)
-            return {0.0, 0.0};
-        const double invd = 1.0 / sqrt(d2);
-        const double d = d2 * invd;
-        const double nxy = -(n[0] * x[0] + n[1] * x[1] + n[2] * x[2]);
-        const cplx<double> e = exp_ik(kap, d);
-        const double f = INV4PI * invd;
-        const double g = kap * (nxy + d); // (g - i) e
-        return {f * (g * e.re + e.im), f * (g * e.im - e.re)};
+        const double d2 = dot3(x, x);
+        const DistInv q = dist_inv<KP::NORMAL>(d2);
+        const double id = d2 < 1e-14 ? 0.0 : q.id;
+        return cmul(cscale(exp_ik(p, q.d), id), cplx<double>{p.kr * (q.d - dot3(n, x)), -1.0});
     }
     __device__ static cplx<double> cf(const double* x, const KParams& p)
     {
-        const double d = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-        return cscale(exp_ik(p.kr, d), INV4PI);
+        return cscale(exp_ik(p, dist_inv<false>(dot3(x, x)).d), INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
-        return exp_ik(p.kr, sqrt(d2) - sqrt(dp2));
+        return exp_ik(p, sqrt(d2) - sqrt(dp2));
     }
-    __device__ static cplx<double> factored(const double* a, const double* n, cplx<double> w,
-                                            const double*, double dc, const KParams& p)
+    __device__ static double leaf_scale(double) { return 1.0; }
+    template <class KP>
+    __device__ static void leaf_add(cplx<double>& s, const double* a, const double* n,
+                                    cplx<double> w, double dc, const KP& p)
     {
-        const double d2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
-        if (!(d2 > 1e-14))
-            return {0.0, 0.0};
-        const double kap = p.kr;
-        const double nxy = -(a[0] * n[0] + a[1] * n[1] + a[2] * n[2]);
-        const double invd = 1.0 / sqrt(d2);
-        const double d = d2 * invd;
-        const cplx<double> v = cmul(w, exp_ik(kap, d - dc));
-        const double g = kap * (nxy + d);
-        return {invd * (g * v.re + v.im), invd * (g * v.im - v.re)};
+        const double d2 = dot3(a, a);
+        const DistInv q = dist_inv<KP::NORMAL>(d2);
+        const double id = d2 > 1e-14 ? q.id : 0.0;
+        cfma(s, w, cmul(cscale(exp_ik(p, q.d - dc), id),
+                        cplx<double>{p.kr * (q.d - dot3(a, n)), -1.0}));
     }
 };
 

@@ -127,85 +127,111 @@ __device__ __forceinline__ void node_position(const LevelGeom& G, int el, int n,
     interp_to_cart(s, xc, H, y);
 }
 
-// One CTA per coarse cone of a leaf box: sum over the leaf's sources
-// (staged in shared memory) at NPT nodes per thread.
+// One CTA per coarse cone of a leaf box (blockIdx.y: chunk of its nodes): sum
+// over the leaf's sources, staged in shared memory, at NPT nodes per thread
+// that share each source's loads.  Bound by the FP64 pipe (about 42 of its
+// instructions per evaluation, issued at three quarters of the 57 FMAs per
+// clock and SM that a loop of independent FMAs reaches): at N = 1e6, p = 9
+// 27.0 ms per matvec with the library functions, 17.9 with the forms of
+// device_math.cuh.  Three CTAs of 256 threads per SM (80 registers): two ran
+// 20.2 ms; one node per thread 21.1, four at 182 registers 20.1.
 template <int KIND>
-__global__ void __launch_bounds__(NODE_THREADS) leaf_sample_kernel(LeafArgs a)
+__global__ void __launch_bounds__(NODE_THREADS, 3) leaf_sample_kernel(LeafArgs a)
 {
     using P = Plugin<KIND>;
-    extern __shared__ double sm[];
+    // per source (x, y), (z, Re w), (Im w, n0), (n1, n2)
+    constexpr int ROWS = P::needs_normals ? 4 : 3;
+    extern __shared__ __align__(16) double2 leaf_sh[];
     const int c = a.idx[blockIdx.x];
     const int node0 = blockIdx.y * NPT * blockDim.x; // node chunk of this CTA
     const int box = a.cc_box[c], el = a.cc_el[c];
     const double xc[3] = {a.T.box_c[3 * box], a.T.box_c[3 * box + 1], a.T.box_c[3 * box + 2]};
     const double H = a.T.box_H[box];
+    const KParamsRegs kp(a.kp);
+    const int nt = blockDim.x;
+    const int f = a.T.box_first[box], l = a.T.box_last[box];
+    // a chunk's source of this thread; the first chunk's loads run ahead of
+    // the node positions
+    double2 v0, v1, v2, v3;
+    auto fetch = [&](int cs) {
+        const int i = cs + (int)threadIdx.x;
+        if (i < l)
+        {
+            const double2 wv = a.w[i];
+            v0 = make_double2(a.S.sx[i], a.S.sy[i]);
+            v1 = make_double2(a.S.sz[i], wv.x);
+            v2 = make_double2(wv.y, P::needs_normals ? a.S.nx[i] : 0.0);
+            if (P::needs_normals)
+                v3 = make_double2(a.S.ny[i], a.S.nz[i]);
+        }
+    };
+    fetch(f);
     double y[NPT][3], dc[NPT];
     cplx<double> acc[NPT];
 #pragma unroll
     for (int q = 0; q < NPT; q++)
     {
-        const int n = node0 + threadIdx.x + q * blockDim.x;
+        // threads past the last node repeat it and write nothing
+        const int n = min(node0 + (int)threadIdx.x + q * (int)blockDim.x, a.P_hi - 1);
         acc[q] = {0.0, 0.0};
-        y[q][0] = y[q][1] = y[q][2] = 0;
-        dc[q] = 0;
-        if (n < a.P_hi)
-        {
-            node_position(a.G, el, n, a.hi_nodes, xc, H, y[q]);
-            const double e0 = y[q][0] - xc[0], e1 = y[q][1] - xc[1], e2 = y[q][2] - xc[2];
-            dc[q] = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
-        }
+        node_position(a.G, el, n, a.hi_nodes, xc, H, y[q]);
+        const double e0 = y[q][0] - xc[0], e1 = y[q][1] - xc[1], e2 = y[q][2] - xc[2];
+        dc[q] = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
     }
-    const int nt = blockDim.x;
-    double* xs = sm;
-    double* ys = xs + nt;
-    double* zs = ys + nt;
-    double* wr = zs + nt;
-    double* wi = wr + nt;
-    double* n0 = wi + nt;
-    double* n1 = n0 + nt;
-    double* n2 = n1 + nt;
-    const int f = a.T.box_first[box], l = a.T.box_last[box];
     for (int cs = f; cs < l; cs += nt)
     {
         const int cnt = min(nt, l - cs);
-        __syncthreads();
+        if (cs != f)
+        {
+            fetch(cs);
+            __syncthreads(); // the previous chunk is no longer read
+        }
         if (threadIdx.x < cnt)
         {
-            const int i = cs + threadIdx.x;
-            xs[threadIdx.x] = a.S.sx[i];
-            ys[threadIdx.x] = a.S.sy[i];
-            zs[threadIdx.x] = a.S.sz[i];
-            const double2 wv = a.w[i];
-            wr[threadIdx.x] = wv.x;
-            wi[threadIdx.x] = wv.y;
+            double2* s = leaf_sh + ROWS * threadIdx.x;
+            s[0] = v0;
+            s[1] = v1;
+            s[2] = v2;
             if (P::needs_normals)
-            {
-                n0[threadIdx.x] = a.S.nx[i];
-                n1[threadIdx.x] = a.S.ny[i];
-                n2[threadIdx.x] = a.S.nz[i];
-            }
+                s[ROWS - 1] = v3;
         }
         __syncthreads();
-#pragma unroll
-        for (int q = 0; q < NPT; q++)
+        for (int i = 0; i < cnt; i++)
         {
-            if (node0 + threadIdx.x + q * blockDim.x >= a.P_hi)
-                continue;
-            for (int i = 0; i < cnt; i++)
+            const double2* s = leaf_sh + ROWS * i;
+            const double2 s0 = s[0], s1 = s[1], s2 = s[2];
+            const double2 s3 = P::needs_normals ? s[ROWS - 1] : make_double2(0.0, 0.0);
+            const double nv[3] = {s2.y, s3.x, s3.y};
+            double av[NPT][3];
+            bool tiny = false;
+#pragma unroll
+            for (int q = 0; q < NPT; q++)
             {
-                const double av[3] = {xs[i] - y[q][0], ys[i] - y[q][1], zs[i] - y[q][2]};
-                const double nv[3] = {P::needs_normals ? n0[i] : 0.0, P::needs_normals ? n1[i] : 0.0,
-                                      P::needs_normals ? n2[i] : 0.0};
-                acc[q] = cadd(acc[q], P::factored(av, nv, {wr[i], wi[i]}, y[q], dc[q], a.kp));
+                av[q][0] = s0.x - y[q][0];
+                av[q][1] = s0.y - y[q][1];
+                av[q][2] = s1.x - y[q][2];
+                tiny |= tiny_square(av[q][0] * av[q][0] + av[q][1] * av[q][1] +
+                                    av[q][2] * av[q][2]);
             }
+            if (!tiny)
+            {
+#pragma unroll
+                for (int q = 0; q < NPT; q++)
+                    P::leaf_add(acc[q], av[q], nv, {s1.y, s2.x}, dc[q], kp);
+            }
+            else
+#pragma unroll
+                for (int q = 0; q < NPT; q++)
+                    P::leaf_add(acc[q], av[q], nv, {s1.y, s2.x}, dc[q], a.kp);
         }
     }
 #pragma unroll
     for (int q = 0; q < NPT; q++)
     {
         const int n = node0 + threadIdx.x + q * blockDim.x;
+        const double f = P::leaf_scale(dc[q]);
         if (n < a.P_hi)
-            a.cvals[(size_t)c * a.P_hi + n] = make_double2(acc[q].re, acc[q].im);
+            a.cvals[(size_t)c * a.P_hi + n] = make_double2(f * acc[q].re, f * acc[q].im);
     }
 }
 
@@ -672,7 +698,7 @@ __global__ void __launch_bounds__(EVAL_THREADS) target_eval_kernel(EvalArgs a)
                         const double nv[3] = {P::needs_normals ? n0[i] : 0.0,
                                               P::needs_normals ? n1[i] : 0.0,
                                               P::needs_normals ? n2[i] : 0.0};
-                        cfma(acc, cplx<double>{wr[i], wi[i]}, P::kernel(x, nv, a.kp));
+                        cfma(acc, cplx<double>{wr[i], wi[i]}, P::kernel4pi(x, nv, a.kp));
                     }
             }
         }
@@ -712,7 +738,7 @@ __global__ void __launch_bounds__(EVAL_THREADS) target_eval_kernel(EvalArgs a)
                 sim += ri[ti + s * cnt];
             }
             if (PART == EVAL_NEAR)
-                a.unear[t] = make_double2(sr, sim);
+                a.unear[t] = make_double2(INV4PI * sr, INV4PI * sim);
             else
             {
                 const double2 nr = a.unear[t];
@@ -751,7 +777,7 @@ __global__ void __launch_bounds__(256) direct_eval_kernel(SrcArgs S, const doubl
         const double x[3] = {S.sx[s] - y0, S.sy[s] - y1, S.sz[s] - y2};
         const double nv[3] = {P::needs_normals ? S.nx[s] : 0.0, P::needs_normals ? S.ny[s] : 0.0,
                               P::needs_normals ? S.nz[s] : 0.0};
-        const cplx<double> g = P::kernel(x, nv, kp);
+        const cplx<double> g = cscale(P::kernel4pi(x, nv, kp), INV4PI);
         const double2 wv = w[s];
         const double vr = wv.x * g.re - wv.y * g.im, vi = wv.x * g.im + wv.y * g.re;
         double yr = vr - cr, tr = ar + yr;
@@ -2143,9 +2169,10 @@ __global__ void __launch_bounds__(PART == EVAL_FAR ? FAR_THREADS : EVAL_THREADS,
 // NODE_THREADS) and the number of node chunks (grid.y) covering P_hi nodes
 inline int node_threads(int P_hi)
 {
-    int t = (P_hi + NPT - 1) / NPT;
-    t = (t + 31) / 32 * 32;
-    return t < 32 ? 32 : (t > NODE_THREADS ? NODE_THREADS : t);
+    // nodes spread evenly over as few chunks as NODE_THREADS allows
+    const int chunks = (P_hi + NPT * NODE_THREADS - 1) / (NPT * NODE_THREADS);
+    const int t = (P_hi + NPT * chunks - 1) / (NPT * chunks);
+    return t < 32 ? 32 : (t + 31) / 32 * 32;
 }
 inline int node_chunks(int P_hi)
 {
@@ -2459,9 +2486,10 @@ __global__ void __launch_bounds__(256) order_probe_kernel(ProbeArgs a)
         const double nv[3] = {P::needs_normals ? a.S.nx[i] : 0.0,
                               P::needs_normals ? a.S.ny[i] : 0.0,
                               P::needs_normals ? a.S.nz[i] : 0.0};
-        acc = cadd(acc, P::factored(av, nv, {1.0, 0.0}, y, dc, a.kp));
+        P::leaf_add(acc, av, nv, {1.0, 0.0}, dc, a.kp);
     }
-    a.out[n] = make_double2(acc.re, acc.im);
+    const double f = P::leaf_scale(dc);
+    a.out[n] = make_double2(f * acc.re, f * acc.im);
 }
 
 template <int KIND>
