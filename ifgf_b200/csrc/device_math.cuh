@@ -395,7 +395,7 @@ __device__ __forceinline__ cplx<double> cheb_eval3(const double2* __restrict__ c
 // Kernel plug-ins.  x = x_src - y_tgt throughout, as in the reference's
 // evaluateKernel loops (e.g. helmholtz_ifgf.hpp:104-111).
 //   kernel4pi  4 pi G
-//   cf         centred factor G(y, xc) (its modulus without the kernel's order)
+//   cf         centred factor G(y, xc) at distance q
 //   transfer   centre shift G(y, x_child) / G(y, x_parent)
 //   leaf_add   s += w G(y, x) / G(y, xc) / leaf_scale(dc) with a = x - y and
 //              dc = |y - xc|: the factor that depends on the node alone is
@@ -425,9 +425,9 @@ template <> struct Plugin<K_LAPLACE>
         const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
         return {!KP::NORMAL && q.d == 0 ? 0.0 : q.id, 0.0};
     }
-    __device__ static cplx<double> cf(const double* x, const KParams&)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams&)
     {
-        return {dist_inv<false>(dot3(x, x)).id * INV4PI, 0.0};
+        return {q.id * INV4PI, 0.0};
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams&)
     {
@@ -453,9 +453,8 @@ template <> struct Plugin<K_HELMHOLTZ>
         const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
         return cscale(exp_ik(p, q.d), !KP::NORMAL && q.d == 0 ? 0.0 : q.id);
     }
-    __device__ static cplx<double> cf(const double* x, const KParams& p)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams& p)
     {
-        const DistInv q = dist_inv<false>(dot3(x, x));
         return cscale(exp_ik(p, q.d), q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
@@ -483,9 +482,8 @@ template <> struct Plugin<K_MODHELMHOLTZ>
         const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
         return exp_mk(p, q.d, !KP::NORMAL && q.d == 0 ? 0.0 : q.id);
     }
-    __device__ static cplx<double> cf(const double* x, const KParams& p)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams& p)
     {
-        const DistInv q = dist_inv<false>(dot3(x, x));
         return exp_mk(p, q.d, q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
@@ -518,9 +516,8 @@ template <> struct Plugin<K_GRADHELMHOLTZ>
         const double f = (id * id) * component(x, p.dx);
         return cmul(exp_mk(p, q.d, f), cplx<double>{p.kr + id, p.ki});
     }
-    __device__ static cplx<double> cf(const double* x, const KParams& p)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams& p)
     {
-        const DistInv q = dist_inv<false>(dot3(x, x));
         return exp_mk(p, q.d, q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
@@ -559,9 +556,8 @@ template <> struct Plugin<K_DOUBLELAYER>
         const double f = (id * id) * dot3(x, n);
         return cmul(exp_mk(p, q.d, f), cplx<double>{p.kr + id, p.ki});
     }
-    __device__ static cplx<double> cf(const double* x, const KParams& p)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams& p)
     {
-        const DistInv q = dist_inv<false>(dot3(x, x));
         return exp_mk(p, q.d, q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
@@ -598,9 +594,8 @@ template <> struct Plugin<K_COMBINEDFIELD>
         return cmul(cscale(exp_ik(p, d), id * id * id),
                     cplx<double>{nxy, -p.kr * fma(d, nxy, d2)});
     }
-    __device__ static cplx<double> cf(const double* x, const KParams& p)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams& p)
     {
-        const DistInv q = dist_inv<false>(dot3(x, x));
         return cscale(exp_ik(p, q.d), q.id * INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
@@ -638,9 +633,9 @@ template <> struct Plugin<K_HELMHOLTZ_DK>
         const bool zero = !KP::NORMAL && d == 0;
         return {zero ? 0.0 : -e.im, zero ? 0.0 : e.re};
     }
-    __device__ static cplx<double> cf(const double* x, const KParams& p)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams& p)
     {
-        return cscale(exp_ik(p, dist_inv<false>(dot3(x, x)).d), INV4PI);
+        return cscale(exp_ik(p, q.d), INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {
@@ -670,9 +665,9 @@ template <> struct Plugin<K_COMBINEDFIELD_DK>
         const double id = d2 < 1e-14 ? 0.0 : q.id;
         return cmul(cscale(exp_ik(p, q.d), id), cplx<double>{p.kr * (q.d - dot3(n, x)), -1.0});
     }
-    __device__ static cplx<double> cf(const double* x, const KParams& p)
+    __device__ static cplx<double> cf(const DistInv& q, const KParams& p)
     {
-        return cscale(exp_ik(p, dist_inv<false>(dot3(x, x)).d), INV4PI);
+        return cscale(exp_ik(p, q.d), INV4PI);
     }
     __device__ static cplx<double> transfer(double d2, double dp2, const KParams& p)
     {

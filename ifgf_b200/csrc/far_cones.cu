@@ -1,0 +1,310 @@
+// Builds the far-cone plan and sums its values per target.
+#include <algorithm>
+#include <chrono>
+#include <cmath>
+#include <cub/cub.cuh>
+
+#include "far_cones.hpp"
+
+namespace ifgf
+{
+
+void FarConePlan::release()
+{
+    mem.release();
+    p = FarConePtrs();
+    pairs = places = 0;
+    ready = refused = captured = false;
+}
+
+namespace
+{
+
+constexpr int THREADS = 256;
+
+// One CTA per target leaf, one thread per (far box, target) pair: the pair's
+// fine cone (the FP64 lookup that marked the active cones,
+// ifgfoperator.hpp:1736-1891), its index in pos, and the pairs of every cone
+// counted, lanes of one cone together.
+__global__ void __launch_bounds__(THREADS)
+    count_kernel(const LevelGeom* __restrict__ lv, TreeArgs T, const double* __restrict__ tx,
+                 const double* __restrict__ ty, const double* __restrict__ tz,
+                 const int* __restrict__ fmap, const int* __restrict__ tl_first,
+                 const int* __restrict__ tl_last, const long long* __restrict__ far_off,
+                 const int* __restrict__ far_src, const long long* __restrict__ leaf_off, int* pos,
+                 int* count, unsigned long long* err)
+{
+    const int tl = blockIdx.x;
+    const int t0 = tl_first[tl], cnt = tl_last[tl] - t0;
+    const long long f0 = far_off[tl], n = (far_off[tl + 1] - f0) * cnt, o = leaf_off[tl];
+    for (long long base = 0; base < n; base += THREADS)
+    {
+        const long long q = base + threadIdx.x;
+        int gf = -1;
+        if (q < n)
+        {
+            const int sb = far_src[f0 + q / cnt], t = t0 + (int)(q % cnt);
+            const LevelGeom& G = lv[T.box_level[sb]];
+            double s[3];
+            cart_to_interp(tx[t] - T.box_c[3 * sb], ty[t] - T.box_c[3 * sb + 1],
+                           tz[t] - T.box_c[3 * sb + 2], T.box_H[sb], s);
+            const int fe = element_for_point(s, G.dmin, G.dmax, G.hfi, G.nf);
+            if (fe >= 0)
+            {
+                const long long nft = (long long)G.nf[0] * G.nf[1] * G.nf[2];
+                gf = fmap[G.fmap_off + (long long)(sb - G.box_off) * nft + fe];
+                if (gf < 0)
+                    atomicAdd(err, 1ull);
+            }
+            pos[o + q] = gf;
+        }
+        const unsigned same = __match_any_sync(~0u, gf);
+        if (gf >= 0 && (threadIdx.x & 31) == __ffs(same) - 1)
+            atomicAdd(count + gf, __popc(same));
+    }
+}
+
+// Places every pair in its cone's list (cursor: next free entry of each
+// cone): its target in tgt, its place in pos.  Targets of one warp that
+// share a cone stay in order and adjacent.
+__global__ void __launch_bounds__(THREADS)
+    place_kernel(const int* __restrict__ tl_first, const int* __restrict__ tl_last,
+                 const long long* __restrict__ far_off, const long long* __restrict__ leaf_off,
+                 int* pos, int* cursor, int* tgt)
+{
+    const int tl = blockIdx.x, lane = threadIdx.x & 31;
+    const int t0 = tl_first[tl], cnt = tl_last[tl] - t0;
+    const long long n = (far_off[tl + 1] - far_off[tl]) * cnt, o = leaf_off[tl];
+    for (long long base = 0; base < n; base += THREADS)
+    {
+        const long long q = base + threadIdx.x;
+        const int gf = q < n ? pos[o + q] : -1;
+        const unsigned same = __match_any_sync(~0u, gf);
+        const int lead = __ffs(same) - 1;
+        int at = 0;
+        if (gf >= 0 && lane == lead)
+            at = atomicAdd(cursor + gf, __popc(same));
+        at = __shfl_sync(~0u, at, lead) + __popc(same & ((1u << lane) - 1));
+        if (gf >= 0)
+        {
+            pos[o + q] = at;
+            tgt[at] = t0 + (int)(q % cnt);
+        }
+    }
+}
+
+// counts rounded up to whole tiles
+__global__ void pad_kernel(int* count, int n)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        count[i] = (count[i] + FAR_TILE - 1) / FAR_TILE * FAR_TILE;
+}
+
+__global__ void tile_kernel(const int* __restrict__ off, int n, int* tile_cone)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        for (int k = off[i] / FAR_TILE; k < off[i + 1] / FAR_TILE; k++)
+            tile_cone[k] = i;
+}
+
+__global__ void meta_kernel(const int* __restrict__ box, const int* __restrict__ el, int n,
+                            int2* meta)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        meta[i] = make_int2(box[i], el[i]);
+}
+
+unsigned blocks_for(long long n)
+{
+    return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, 148 * 32));
+}
+
+} // namespace
+
+void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
+{
+    const auto start = std::chrono::steady_clock::now();
+    plan.release();
+    const std::vector<LevelGeom>& lv = *b.lv;
+    const int L = (int)lv.size(), nl = b.n_tleaf;
+    long long n_fine = 0;
+    for (const LevelGeom& G : lv)
+        n_fine += G.n_fine;
+    const long long pairs = b.leaf_off->back();
+    // places at most: every cone with pairs wastes less than a tile
+    const long long most =
+        (pairs + (FAR_TILE - 1) * std::min(n_fine, pairs) + 31) / 32 * 32;
+    if (pairs <= 0 || n_fine <= 0 || most >= (1ll << 31) - 1)
+    {
+        plan.refused = true;
+        return;
+    }
+    // host tables: leaf offsets; sines and cosines of the centre angles of
+    // every level's fine cones
+    std::vector<double2> trig;
+    std::vector<int2> level(L);
+    for (int l = 0; l < L; l++)
+    {
+        const LevelGeom& G = lv[l];
+        // narrow: half widths within the range of asin_small
+        level[l] = make_int2((int)trig.size(), std::max(G.hf[1], G.hf[2]) <= 0.525 ? 1 : 0);
+        for (int d = 1; d < 3; d++)
+            for (int i = 0; i < G.nf[d]; i++)
+            {
+                const double c = G.dmin[d] + ((double)i + 0.5) * G.hf[d];
+                trig.push_back(make_double2(std::sin(c), std::cos(c)));
+            }
+    }
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, (int*)nullptr, (int*)nullptr, (int)n_fine + 1);
+    // one allocation; the scratch of the build shares the values' place
+    size_t used_b = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = used_b;
+        used_b += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t cb = ((size_t)(n_fine + 1) * sizeof(int) + 255) / 256 * 256;
+    const size_t o_val = place(std::max((size_t)most * sizeof(double2), 2 * cb + tb));
+    const size_t o_pos = place((size_t)pairs * sizeof(int));
+    const size_t o_tgt = place((size_t)most * sizeof(int));
+    const size_t o_tile = place((size_t)most / FAR_TILE * sizeof(int));
+    const size_t o_meta = place((size_t)n_fine * sizeof(int2));
+    const size_t o_host = used_b;
+    const size_t o_leaf = place(b.leaf_off->size() * sizeof(long long));
+    const size_t o_trig = place(trig.size() * sizeof(double2));
+    const size_t o_lev = place(level.size() * sizeof(int2));
+    if (used_b > (size_t(256) << 20))
+    {
+        size_t free_b = 0, total_b = 0;
+        IFGF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        if (used_b > free_b / 4)
+        {
+            plan.refused = true;
+            return;
+        }
+    }
+    try
+    {
+        plan.mem.alloc(used_b);
+    }
+    catch (const Error&)
+    {
+        plan.refused = true;
+        return;
+    }
+    unsigned char* m = plan.mem.p;
+    std::vector<unsigned char> host(used_b - o_host);
+    std::copy_n((const unsigned char*)b.leaf_off->data(), b.leaf_off->size() * sizeof(long long),
+                host.data() + (o_leaf - o_host));
+    std::copy_n((const unsigned char*)trig.data(), trig.size() * sizeof(double2),
+                host.data() + (o_trig - o_host));
+    std::copy_n((const unsigned char*)level.data(), level.size() * sizeof(int2),
+                host.data() + (o_lev - o_host));
+    IFGF_CUDA(cudaMemcpy(m + o_host, host.data(), host.size(), cudaMemcpyHostToDevice));
+    int* pos = (int*)(m + o_pos);
+    int* tgt = (int*)(m + o_tgt);
+    int* tile = (int*)(m + o_tile);
+    int2* meta = (int2*)(m + o_meta);
+    const long long* leaf_off = (const long long*)(m + o_leaf);
+    int* count = (int*)(m + o_val);
+    int* off = (int*)(m + o_val + cb);
+    IFGF_CUDA(cudaMemsetAsync(count, 0, (n_fine + 1) * sizeof(int), nullptr));
+    IFGF_CUDA(cudaMemsetAsync(tgt, 0xff, o_meta - o_tgt, nullptr)); // and the tiles
+    for (int l = 0; l < L; l++)
+        if (lv[l].n_fine > 0)
+            meta_kernel<<<blocks_for(lv[l].n_fine), 256>>>(b.cone_box[l], b.cone_el[l],
+                                                           (int)lv[l].n_fine,
+                                                           meta + lv[l].fine_off);
+    count_kernel<<<nl, THREADS>>>(b.lv_dev, b.T, b.tx, b.ty, b.tz, b.fmap, b.tl_first, b.tl_last,
+                                  b.far_off, b.far_src, leaf_off, pos, count, b.err);
+    pad_kernel<<<blocks_for(n_fine), 256>>>(count, (int)n_fine);
+    IFGF_CUDA(cub::DeviceScan::ExclusiveSum(m + o_val + 2 * cb, tb, count, off, (int)n_fine + 1));
+    tile_kernel<<<blocks_for(n_fine), 256>>>(off, (int)n_fine, tile);
+    int used = 0;
+    IFGF_CUDA(cudaMemcpy(&used, off + n_fine, sizeof(int), cudaMemcpyDeviceToHost));
+    // off becomes every cone's cursor
+    place_kernel<<<nl, THREADS>>>(b.tl_first, b.tl_last, b.far_off, leaf_off, pos, off, tgt);
+    IFGF_CUDA(cudaGetLastError());
+    IFGF_CUDA(cudaDeviceSynchronize());
+    if (used == 0) // every pair outside its box's domain
+    {
+        plan.release();
+        plan.refused = true;
+        return;
+    }
+    plan.pairs = pairs;
+    plan.places = ((long long)used + 31) / 32 * 32;
+    plan.p = FarConePtrs{tile, plan.places / 32, tgt,      meta,
+                         (const int2*)(m + o_lev),   (const double2*)(m + o_trig),
+                         pos,  leaf_off,             (double2*)(m + o_val)};
+    plan.ready = true;
+    plan.ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - start)
+                  .count();
+}
+
+// One CTA per target leaf: thread (ti, si) adds the values of target ti over
+// far boxes si, si + S, ... (S = threads / targets); the S sums and the near
+// sum are added in a fixed order and written in the caller's order.  Bound
+// by memory (20 bytes a pair).
+__global__ void __launch_bounds__(THREADS)
+    far_gather_kernel(FarConePtrs fc, const int* __restrict__ tl_first,
+                      const int* __restrict__ tl_last, const long long* __restrict__ far_off,
+                      const double2* __restrict__ unear, const long long* __restrict__ tgt_perm,
+                      double* out, int real_out)
+{
+    __shared__ double2 part[THREADS];
+    const int tl = blockIdx.x;
+    const int t0 = tl_first[tl], all = tl_last[tl] - t0;
+    const int nbox = (int)(far_off[tl + 1] - far_off[tl]);
+    for (int base = 0; base < all; base += THREADS)
+    {
+        const int cnt = min(THREADS, all - base);
+        const int S = THREADS / cnt;
+        const int ti = threadIdx.x % cnt, si = threadIdx.x / cnt;
+        double2 acc = make_double2(0.0, 0.0);
+        if (si < S)
+        {
+            const int* pos = fc.pos + fc.leaf_off[tl] + base + ti;
+#pragma unroll 4
+            for (int e = si; e < nbox; e += S)
+            {
+                const int at = pos[(long long)e * all];
+                if (at >= 0)
+                {
+                    const double2 v = fc.val[at];
+                    acc.x += v.x;
+                    acc.y += v.y;
+                }
+            }
+        }
+        __syncthreads(); // the previous chunk's sums are no longer read
+        part[threadIdx.x] = acc;
+        __syncthreads();
+        if (si == 0)
+        {
+            for (int s = 1; s < S; s++)
+            {
+                acc.x += part[ti + s * cnt].x;
+                acc.y += part[ti + s * cnt].y;
+            }
+            const double2 nr = unear[t0 + base + ti];
+            acc.x += nr.x;
+            acc.y += nr.y;
+            const long long o = tgt_perm[t0 + base + ti];
+            if (real_out)
+                out[o] = acc.x;
+            else
+                reinterpret_cast<double2*>(out)[o] = acc;
+        }
+    }
+}
+
+void launch_far_gather(const MultPtrs& m, void* d_u, bool real, cudaStream_t st)
+{
+    far_gather_kernel<<<m.n_tleaf, THREADS, 0, st>>>(m.fc, m.tl_first, m.tl_last, m.tl_far_off,
+                                                     m.unear, m.tgt_perm, (double*)d_u,
+                                                     real ? 1 : 0);
+}
+
+} // namespace ifgf

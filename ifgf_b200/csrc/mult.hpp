@@ -118,6 +118,22 @@ void launch_build_upgeo(const LevelGeom& PG, const LevelGeom& CG, double pH, dou
                         const double* hi_nodes, int P_hi, KParams kp, int P_pad, UpGeo64* g64,
                         UpGeo32* g32, int fe_pad, int2* fe_list);
 
+// Far-cone plan (far_cones.hpp) as the kernels see it: the (target, far box)
+// pairs sorted by fine cone, each cone's padded to whole tiles of FAR_TILE.
+constexpr int FAR_TILE = 8;
+struct FarConePtrs
+{
+    const int* tile_cone = nullptr; // cone of every tile, -1 past the last; null: no plan
+    long long n_groups = 0;         // groups of 32 places (4 tiles)
+    const int* tgt = nullptr;       // target of every place, -1 for padding
+    const int2* meta = nullptr;     // (box, fine element) of every cone
+    const int2* level = nullptr;    // per level: first trig entry, narrow cones
+    const double2* trig = nullptr;  // per level (sin, cos) of the theta, then the phi centres
+    const int* pos = nullptr;       // per target leaf [far box][target]: place, or -1
+    const long long* leaf_off = nullptr; // first pos entry of every target leaf
+    double2* val = nullptr;         // value of every place
+};
+
 // Everything one matvec launch needs (device pointers, sizes, orders).
 struct MultPtrs
 {
@@ -162,9 +178,14 @@ struct MultPtrs
     // the upward-kernel autotuner's per-level choice for single-plane
     // matvecs (host array of L: 1 tensor cores, 0 FFMA, -1 none yet)
     const signed char* up_choice = nullptr;
+    // far-cone plan of the FP64 far field (null: the
+    // far kernel looks up every pair's cone)
+    FarConePtrs fc;
 };
 
-
+// Sums of a far-cone plan's values per target, plus the near sums, into the
+// caller's result (far_cones.cu).
+void launch_far_gather(const MultPtrs& m, void* d_u, bool real, cudaStream_t st);
 
 // Stage classes for per-kernel timing.
 enum ProfClass

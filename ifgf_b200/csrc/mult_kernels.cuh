@@ -723,7 +723,7 @@ __global__ void __launch_bounds__(EVAL_THREADS) target_eval_kernel(EvalArgs a)
                 }
                 to_local(fe, s, G.dmin, G.hf, G.hfi, G.nf, loc);
                 const cplx<double> v = Cheb<N0, N1, N2>::eval(a.fcoef + (size_t)gf * a.P_lo, loc, a.lo);
-                cfma(acc, v, P::cf(p, a.kp));
+                cfma(acc, v, P::cf(dist_inv<false>(dot3(p, p)), a.kp));
             }
         __syncthreads();
         rr[threadIdx.x] = acc.re;
@@ -2181,6 +2181,7 @@ inline int node_chunks(int P_hi)
 }
 
 #include "far_staged.cuh"
+#include "far_cones.cuh"
 
 template <int KIND, int N0, int N1, int N2, bool MIXED>
 static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cudaStream_t st,
@@ -2414,11 +2415,26 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
     }
     if (m.n_tleaf > 0)
     {
-        if (overlap)
-            IFGF_CHECK(cudaStreamWaitEvent(st, m.ev_join, 0));
         if (hk)
             hk->begin(PROF_EVAL);
-        if (MIXED)
+        bool by_cone = false;
+        if constexpr (!MIXED && N0 > 0)
+            if (m.fc.tile_cone)
+            {
+                const FarConeArgs fa{m.fc, m.lv_dev, m.T, m.tx, m.ty, m.tz, m.fcoef, m.kp};
+                constexpr int WARPS = FAR_CONE_THREADS / 32;
+                far_cone_kernel<KIND, N0, N1, N2>
+                    <<<(unsigned)((m.fc.n_groups - 1) / WARPS + 1), FAR_CONE_THREADS, 0, st>>>(fa);
+                IFGF_CHECK_LAUNCH();
+                launches++;
+                by_cone = true;
+            }
+        // the near sums are read from here on
+        if (overlap)
+            IFGF_CHECK(cudaStreamWaitEvent(st, m.ev_join, 0));
+        if (by_cone)
+            launch_far_gather(m, d_u, real, st);
+        else if (MIXED)
             target_eval_mixed_kernel<KIND, N0, N1, N2, EVAL_FAR><<<m.n_tleaf, FAR_THREADS, 0, st>>>(ea);
         else
             target_eval_kernel<KIND, N0, N1, N2, EVAL_FAR><<<m.n_tleaf, EVAL_THREADS, 0, st>>>(ea);

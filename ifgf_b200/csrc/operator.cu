@@ -12,6 +12,7 @@
 
 #include "devbuf.hpp"
 #include "device_math.cuh"
+#include "far_cones.hpp"
 #include "gpu_target_lists.hpp"
 #include "tcgen05.cuh"
 #include "mult.hpp"
@@ -73,6 +74,8 @@ struct DeviceState
     double fp_ovf_few = 0; // share of the records beyond the smaller slot count tried
     bool fp_ready = false;
     double fp_ms = 0;
+    FarConePlan fc; // far-cone plan of the FP64 matvec
+    std::vector<long long> tl_pair_off; // first (far box, target) pair of every target leaf
     DevBuf<double2> w, cvals, fcoef, unear;
     // planes of the batched mixed matvec, allocated on first use for
     // b_planes planes of the plane sizes recorded beside them
@@ -1225,11 +1228,20 @@ void Operator::setup_device(const double* normals)
         }
         D.tl_first.upload(f);
         D.tl_last.upload(l);
+        D.tl_pair_off.assign(ntl + 1, 0);
+        for (int64_t i = 0; i < ntl; i++)
+            D.tl_pair_off[i + 1] = l[i] - f[i]; // targets for now
         D.n_tleaf = (int)ntl;
     }
     phase("boxes_points_upload");
     build_target_lists_gpu(plan_, shard_n_ > 1 ? shard_rank_ : -1, D.tl_far_off, D.tl_far_src,
                            D.tl_near_off, D.tl_near_src);
+    {
+        const std::vector<long long> fo = D.tl_far_off.download();
+        for (int i = 0; i < D.n_tleaf; i++)
+            D.tl_pair_off[i + 1] =
+                D.tl_pair_off[i] + D.tl_pair_off[i + 1] * (fo[i + 1] - fo[i]);
+    }
     // the far-field plan of earlier tables is stale: rebuilt on first use
     D.fp_chunk.release();
     D.fp_group.release();
@@ -1237,6 +1249,7 @@ void Operator::setup_device(const double* normals)
     D.fp_slot.release();
     D.fp_nchunk = 0;
     D.fp_ready = false;
+    D.fc.release();
     phase("target_leaf_lists");
     // ---- active cones (octree.hpp:351-816) on the GPU ----
     int64_t fmap_total = 0;
@@ -1760,7 +1773,54 @@ void Operator::set_far_plan(bool on)
         D.fp_slot.release();
         D.fp_nchunk = 0;
         D.fp_ready = false;
+        // a captured graph may still read the far-cone plan: kept until the
+        // next init
+        if (!D.fc.captured)
+            D.fc.release();
     }
+}
+
+void Operator::ensure_far_cones(MultPtrs& m, void* stream)
+{
+    DeviceState& D = *dev_;
+    if (!far_plan_on_ || D.n_tleaf == 0)
+        return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess)
+    {
+        cudaGetLastError();
+        cap = cudaStreamCaptureStatusActive;
+    }
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    if (!D.fc.ready && !D.fc.refused && !capturing)
+    {
+        IFGF_CUDA(cudaSetDevice(device_));
+        FarConeBuild b;
+        b.lv = &lv_;
+        b.lv_dev = D.lv.p;
+        b.T = m.T;
+        b.tx = D.tx.p;
+        b.ty = D.ty.p;
+        b.tz = D.tz.p;
+        b.fmap = D.fmap.p;
+        b.tl_first = D.tl_first.p;
+        b.tl_last = D.tl_last.p;
+        b.far_off = D.tl_far_off.p;
+        b.leaf_off = &D.tl_pair_off;
+        b.far_src = D.tl_far_src.p;
+        b.n_tleaf = D.n_tleaf;
+        for (size_t l = 0; l < lv_.size(); l++)
+        {
+            b.cone_box.push_back(D.fc_box[l].p);
+            b.cone_el.push_back(D.fc_el[l].p);
+        }
+        b.err = D.err.p;
+        build_far_cones(b, D.fc);
+    }
+    if (!D.fc.ready)
+        return;
+    D.fc.captured |= capturing;
+    m.fc = D.fc.p;
 }
 
 void Operator::ensure_far_plan()
@@ -2276,6 +2336,8 @@ void Operator::launch_mult(const void* d_w, void* d_u, void* stream, bool timed,
     }
     MultPtrs m;
     fill_mult_ptrs(m, vkind >= 0);
+    if (precision_ == PREC_FP64)
+        ensure_far_cones(m, stream);
     EventHooks log(D, st);
     const bool on = profiling_ || timed;
     int launches = 0;
@@ -2890,6 +2952,9 @@ std::string Operator::stats_json() const
       << (dev_->fp_group.n * sizeof(FarGroup) + dev_->fp_rec.n * sizeof(FarPlanRec) +
           dev_->fp_slot.n * sizeof(int) + dev_->fp_chunk.n * sizeof(FarChunk))
       << ",\"slots_per_group\":" << dev_->fp_nslot << ",\"overflow_share_at_few_slots\":" << dev_->fp_ovf_few << ",\"build_ms\":" << dev_->fp_ms << "}";
+    o << ",\"far_cones\":{\"built\":" << (dev_->fc.ready ? 1 : 0)
+      << ",\"pairs\":" << dev_->fc.pairs << ",\"places\":" << dev_->fc.places
+      << ",\"bytes\":" << dev_->fc.mem.n << ",\"build_ms\":" << dev_->fc.ms << "}";
     o << ",\"upward_images_bytes\":[";
     for (int l = 0; l < (int)lv_.size(); l++)
         o << (l ? "," : "") << (l < (int)dev_->tc_img.size() ? dev_->tc_img[l].n : 0);
