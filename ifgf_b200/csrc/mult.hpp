@@ -187,6 +187,29 @@ struct MultPtrs
 // caller's result (far_cones.cu).
 void launch_far_gather(const MultPtrs& m, void* d_u, bool real, cudaStream_t st);
 
+struct C2FArgs
+{
+    LevelGeom G;
+    const int* __restrict__ idx; // coarse cones to refine (null: all of the level)
+    // batched right-hand sides (fixed-order kernel): blockIdx.y selects the plane
+    long long cv_plane, fc_plane;
+    const int* __restrict__ cc_box;
+    const int* __restrict__ cc_el;
+    const double2* __restrict__ cvals;
+    const double* __restrict__ A; // A0 | A1 | A2, row-major (f_d lo_d) x ho_d
+    const int* __restrict__ fmap;
+    double2* fcoef;
+    int hi[3], lo[3], f[3];
+    int P_hi, P_lo;
+};
+
+// Fixed-order coarse-to-fine kernels (coarse_to_fine.cu): launch one for the
+// shape (hi, lo, f) of `fa` and return true, or false where none exists.
+// A_host: the three matrices.  FP32 over `planes` planes.
+bool launch_c2f_fixed_f32(const C2FArgs& fa, const double* A_host, unsigned grid, cudaStream_t st,
+                          unsigned planes);
+bool launch_c2f_fixed_f64(const C2FArgs& fa, const double* A_host, unsigned grid, cudaStream_t st);
+
 // Stage classes for per-kernel timing.
 enum ProfClass
 {

@@ -534,7 +534,7 @@ static int run_mult_batch(const MultPtrs& m, const BatchPtrs& bp, const void* d_
             fa.P_lo = m.P_lo;
             if (hk)
                 hk->begin(PROF_C2F, l);
-            if (!launch_c2f_fixed<float>(fa, m.A_host, c2f_grid, st, bp.groups * BATCH_NB))
+            if (!launch_c2f_fixed_f32(fa, m.A_host, c2f_grid, st, bp.groups * BATCH_NB))
                 throw Error(6, "batched coarse-to-fine needs one of the fixed order shapes");
             IFGF_CHECK_LAUNCH();
             if (hk)

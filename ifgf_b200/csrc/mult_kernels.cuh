@@ -502,22 +502,6 @@ void launch_build_upgeo(const LevelGeom& PG, const LevelGeom& CG, double pH, dou
 }
 
 
-struct C2FArgs
-{
-    LevelGeom G;
-    const int* __restrict__ idx; // coarse cones to refine (null: all of the level)
-    // batched right-hand sides (fixed-order kernel): blockIdx.y selects the plane
-    long long cv_plane, fc_plane;
-    const int* __restrict__ cc_box;
-    const int* __restrict__ cc_el;
-    const double2* __restrict__ cvals;
-    const double* __restrict__ A; // A0 | A1 | A2, row-major (f_d lo_d) x ho_d
-    const int* __restrict__ fmap;
-    double2* fcoef;
-    int hi[3], lo[3], f[3];
-    int P_hi, P_lo;
-};
-
 // Coarse nodal values -> fine Chebyshev coefficients of the active sub-cones.
 static __global__ void __launch_bounds__(256) coarse_to_fine_kernel(C2FArgs a)
 {
@@ -1727,267 +1711,6 @@ static __global__ void __launch_bounds__(256) coarse_to_fine_mixed_kernel(C2FArg
     }
 }
 
-// Coarse-to-fine with compile-time orders and refinement factor F (the same
-// in every dimension), for the common order triples.  T is the working
-// precision (double, or float in the mixed pipeline); the three matrices are
-// staged in shared memory in T.
-template <typename T> struct Vec2;
-template <> struct Vec2<double>
-{
-    using type = double2;
-};
-template <> struct Vec2<float>
-{
-    using type = float2;
-};
-
-// The three per-dimension matrices as a kernel parameter: with every loop
-// unrolled, each entry is a compile-time offset into the parameter bank and
-// enters its FMA as a constant operand, so the contraction reads only the
-// data operand from shared memory.
-template <int H0, int H1, int H2, int L0, int L1, int L2, int F, typename T>
-struct C2FMats
-{
-    T a0[F * L0 * H0];
-    T a1[F * L1 * H1];
-    T a2[F * L2 * H2];
-};
-
-// Row stride of the second intermediate: F0 F1 rounded up so that the rows
-// of consecutive m2 start F0 banks apart (conflict-free stage-2 stores).
-template <int F0, int F1>
-__host__ __device__ constexpr int c2f_row_stride()
-{
-    int s = F0 * F1;
-    while (s % 16 != F0 % 16)
-        s++;
-    return s;
-}
-
-// stage 2 of the fixed coarse-to-fine kernel: threads per fine column
-// block j0 (its L0 x H2 row vectors, whole warps, so that a warp works for
-// one j0 only)
-template <int H2, int L0> __host__ __device__ constexpr int c2f_stage2_group()
-{
-    return (L0 * H2 + 31) / 32 * 32;
-}
-
-// one thread per row vector of the widest of the three stages
-template <int H0, int H1, int H2, int L0, int L1, int L2, int F>
-constexpr int c2f_fixed_threads()
-{
-    constexpr int s1 = H1 * H2, s2 = F * c2f_stage2_group<H2, L0>(), s3 = F * L0 * F * L1;
-    constexpr int m = s1 > s2 ? (s1 > s3 ? s1 : s3) : (s2 > s3 ? s2 : s3);
-    return (m + 31) / 32 * 32;
-}
-
-// Coarse-to-fine with compile-time orders and refinement factor F (the same
-// in every dimension), one coarse cone per block, register-tiled: every
-// thread loads one input vector of a mode product into registers once and
-// produces all output rows that use it.
-//   stage 1 (thread = (m1, m2)):  Y1[i0][m1][m2] = sum_m A0[i0][m] X[m][m1][m2]
-//   stage 2 (thread = (i0, m2)):  Y2[m2][i0 + F0 i1] = sum_m A1[i1][m] Y1[i0][m][m2]
-//   stage 3 (thread = i0 + F0 i1): C[j2 L2 + i2] = sum_m A2[j2 L2 + i2][m] Y2[m][.]
-// Stage 3 writes the coefficients of every active sub-cone straight to
-// global memory.  Warps follow the sub-cones: a stage-2 warp works for one
-// fine column block j0 and skips the row blocks j1 whose sub-cones (j0, j1,
-// j2) are all inactive; stage-3 threads go sub-cone by sub-cone (L0 L1 each),
-// so that a warp spans about two sub-cones, skips the j2 where they are
-// inactive and writes each active one's rows as contiguous runs.  NPL
-// planes per CTA (blockIdx.y: planes NPL y ...): each matrix constant, index
-// and barrier then serves NPL row vectors (2 for FP32 batches: 3.15 -> 3.03
-// ms per batched matvec at N = 1e6).  T is the working precision (double,
-// or float in the mixed pipeline).
-template <int H0, int H1, int H2, int L0, int L1, int L2, int F, typename T, int NPL>
-__global__ void __launch_bounds__(c2f_fixed_threads<H0, H1, H2, L0, L1, L2, F>())
-    coarse_to_fine_fixed_kernel(C2FArgs a, const C2FMats<H0, H1, H2, L0, L1, L2, F, T> M)
-{
-    using V = typename Vec2<T>::type;
-    constexpr int F0 = F * L0, F1 = F * L1;
-    constexpr int P_HI = H0 * H1 * H2, P_LO = L0 * L1 * L2;
-    constexpr int S2 = c2f_row_stride<F0, F1>();
-    constexpr int Y1N = F0 * H1 * H2, YN = Y1N + S2 * H2; // elements per plane
-    extern __shared__ __align__(16) unsigned char c2f_raw[];
-    // plane p: Y1 at p YN ([m2][m1][i0], i0 fastest), Y2 at p YN + Y1N ([m2][S2])
-    V* Y = reinterpret_cast<V*>(c2f_raw);
-    __shared__ int gsub[F * F * F];
-    const int c = a.idx ? a.idx[blockIdx.x] : (int)blockIdx.x;
-    const int t = threadIdx.x;
-    const int box = a.cc_box[c], el = a.cc_el[c];
-    const int p0 = blockIdx.y * NPL; // first plane of the CTA
-    if (t < F * F * F)
-    {
-        const int nc0 = a.G.nc[0], nc1 = a.G.nc[1];
-        const int hid0 = el % nc0, hid1 = (el / nc0) % nc1, hid2 = el / (nc0 * nc1);
-        const int nf0 = a.G.nf[0], nf1 = a.G.nf[1];
-        const long long nft = (long long)nf0 * nf1 * a.G.nf[2];
-        const int* fm = a.fmap + a.G.fmap_off + (long long)(box - a.G.box_off) * nft;
-        const int j0 = t % F, j1 = (t / F) % F, j2 = t / (F * F);
-        gsub[t] = fm[((hid2 * F + j2) * nf1 + (hid1 * F + j1)) * nf0 + (hid0 * F + j0)];
-    }
-    if (t < H1 * H2)
-    {
-        V x[NPL][H0];
-#pragma unroll
-        for (int p = 0; p < NPL; p++)
-        {
-            const V* src = reinterpret_cast<const V*>(a.cvals) + (p0 + p) * a.cv_plane +
-                           (size_t)c * P_HI + H0 * t;
-#pragma unroll
-            for (int m = 0; m < H0; m++)
-                x[p][m] = src[m];
-        }
-#pragma unroll
-        for (int i0 = 0; i0 < F0; i0++)
-        {
-#pragma unroll
-            for (int p = 0; p < NPL; p++)
-            {
-                T re = 0, im = 0;
-#pragma unroll
-                for (int m = 0; m < H0; m++)
-                {
-                    re = fma(M.a0[i0 * H0 + m], x[p][m].x, re);
-                    im = fma(M.a0[i0 * H0 + m], x[p][m].y, im);
-                }
-                Y[p * YN + i0 + F0 * t] = V{re, im};
-            }
-        }
-    }
-    __syncthreads();
-    constexpr int G2 = c2f_stage2_group<H2, L0>();
-    if (t < F * G2 && t % G2 < L0 * H2)
-    {
-        const int j0 = t / G2, u = t % G2;
-        const int i0 = j0 * L0 + u % L0, m2 = u / L0;
-        V x[NPL][H1];
-#pragma unroll
-        for (int p = 0; p < NPL; p++)
-#pragma unroll
-            for (int m = 0; m < H1; m++)
-                x[p][m] = Y[p * YN + i0 + F0 * (m + H1 * m2)];
-#pragma unroll
-        for (int j1 = 0; j1 < F; j1++)
-        {
-            bool used = false;
-#pragma unroll
-            for (int j2 = 0; j2 < F; j2++)
-                used |= gsub[j0 + F * (j1 + F * j2)] >= 0;
-            if (!used)
-                continue; // no active sub-cone reads these rows
-#pragma unroll
-            for (int i1 = j1 * L1; i1 < (j1 + 1) * L1; i1++)
-            {
-#pragma unroll
-                for (int p = 0; p < NPL; p++)
-                {
-                    T re = 0, im = 0;
-#pragma unroll
-                    for (int m = 0; m < H1; m++)
-                    {
-                        re = fma(M.a1[i1 * H1 + m], x[p][m].x, re);
-                        im = fma(M.a1[i1 * H1 + m], x[p][m].y, im);
-                    }
-                    Y[p * YN + Y1N + i0 + F0 * i1 + S2 * m2] = V{re, im};
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (t < F0 * F1)
-    {
-        const int q = t % (L0 * L1), sc = t / (L0 * L1);
-        const int i0 = q % L0, i1 = q / L0, j0 = sc % F, j1 = sc / F;
-        const int i0f = j0 * L0 + i0, i1f = j1 * L1 + i1;
-        V x[NPL][H2];
-#pragma unroll
-        for (int p = 0; p < NPL; p++)
-#pragma unroll
-            for (int m = 0; m < H2; m++)
-                x[p][m] = Y[p * YN + Y1N + i0f + F0 * i1f + S2 * m];
-#pragma unroll
-        for (int j2 = 0; j2 < F; j2++)
-        {
-            const int gf = gsub[j0 + F * (j1 + F * j2)];
-            if (gf < 0)
-                continue;
-#pragma unroll
-            for (int i2 = 0; i2 < L2; i2++)
-            {
-#pragma unroll
-                for (int p = 0; p < NPL; p++)
-                {
-                    T re = 0, im = 0;
-#pragma unroll
-                    for (int m = 0; m < H2; m++)
-                    {
-                        re = fma(M.a2[(j2 * L2 + i2) * H2 + m], x[p][m].x, re);
-                        im = fma(M.a2[(j2 * L2 + i2) * H2 + m], x[p][m].y, im);
-                    }
-                    V* fco = reinterpret_cast<V*>(a.fcoef) + (p0 + p) * a.fc_plane;
-                    fco[(size_t)gf * P_LO + i0 + L0 * i1 + L0 * L1 * i2] = V{re, im};
-                }
-            }
-        }
-    }
-}
-
-template <int H0, int H1, int H2, int L0, int L1, int L2, int F, typename T>
-constexpr size_t c2f_fixed_smem(int npl = 1)
-{
-    constexpr int F0 = F * L0, F1 = F * L1;
-    return (size_t)npl * (F0 * H1 * H2 + c2f_row_stride<F0, F1>() * H2) * 2 * sizeof(T);
-}
-
-// Launches the fixed-size coarse-to-fine kernel when (hi, lo, f) is one of the
-// instantiated shapes; returns false otherwise.
-template <typename T>
-static bool launch_c2f_fixed(const C2FArgs& fa, const double* A_host, unsigned grid,
-                             cudaStream_t st, unsigned planes = 1)
-{
-    const int* h = fa.hi;
-    const int* l = fa.lo;
-    const int f = fa.f[0];
-    if (fa.f[1] != f || fa.f[2] != f || (f != 3 && f != 1) || A_host == nullptr)
-        return false;
-    // refinement factor 3 (fine grid 3x the coarse one) or 1 (the modified
-    // Helmholtz kernel: fine = coarse grid)
-#define IFGF_C2F_CASE_F(A, B, C, D, E, G, F)                                                  \
-    {                                                                                          \
-        C2FMats<A, B, C, D, E, G, F, T> mats;                                                  \
-        T* dst = mats.a0;                                                                      \
-        constexpr int NA = F * (D * A + E * B + G * C);                                        \
-        static_assert(sizeof(mats) == NA * sizeof(T), "matrix block layout");                  \
-        for (int i = 0; i < NA; i++)                                                           \
-            dst[i] = (T)A_host[i];                                                             \
-        /* FP32: two planes per CTA share every matrix constant and index */                  \
-        constexpr int NPL = std::is_same<T, float>::value ? 2 : 1;                             \
-        const int npl = planes % NPL == 0 ? NPL : 1;                                           \
-        const size_t sm = c2f_fixed_smem<A, B, C, D, E, G, F, T>(npl);                         \
-        auto kern = npl == 2 ? coarse_to_fine_fixed_kernel<A, B, C, D, E, G, F, T, NPL>        \
-                             : coarse_to_fine_fixed_kernel<A, B, C, D, E, G, F, T, 1>;         \
-        if (sm > 48 * 1024)                                                                    \
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);  \
-        kern<<<dim3(grid, planes / npl), c2f_fixed_threads<A, B, C, D, E, G, F>(), sm, st>>>(  \
-            fa, mats);                                                                         \
-        return true;                                                                           \
-    }
-#define IFGF_C2F_CASE(A, B, C, D, E, G)                                                       \
-    if (h[0] == A && h[1] == B && h[2] == C && l[0] == D && l[1] == E && l[2] == G)            \
-    {                                                                                          \
-        if (f == 3)                                                                            \
-            IFGF_C2F_CASE_F(A, B, C, D, E, G, 3)                                               \
-        else                                                                                   \
-            IFGF_C2F_CASE_F(A, B, C, D, E, G, 1)                                               \
-    }
-    IFGF_C2F_CASE(5, 8, 8, 2, 5, 5)
-    IFGF_C2F_CASE(6, 9, 9, 3, 6, 6)
-    IFGF_C2F_CASE(7, 10, 10, 4, 7, 7)
-#undef IFGF_C2F_CASE
-#undef IFGF_C2F_CASE_F
-    return false;
-}
-
 // Mixed-precision target leaf evaluation: near-field terms in FP32 on
 // coordinates relative to the leaf's first target, far-field Chebyshev sums
 // in FP32, every contribution accumulated in FP64.
@@ -2343,7 +2066,7 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
                     if (sm > 48 * 1024)
                         IFGF_CHECK(cudaFuncSetAttribute(
                             kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                    kern<<<LL.n_up, UPS64_THREADS, sm, st>>>(ua);
+                    kern<<<LL.n_up, ups64_threads(N0 * N1 * N2), sm, st>>>(ua);
                     staged = true;
                 }
             }
@@ -2400,8 +2123,8 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         fa.P_lo = m.P_lo;
         if (hk)
             hk->begin(PROF_C2F, l);
-        if (launch_c2f_fixed<typename std::conditional<MIXED, float, double>::type>(
-                fa, m.A_host, c2f_grid, st))
+        if (MIXED ? launch_c2f_fixed_f32(fa, m.A_host, c2f_grid, st, 1)
+                  : launch_c2f_fixed_f64(fa, m.A_host, c2f_grid, st))
         {
         }
         else if (MIXED)
@@ -2437,7 +2160,12 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         else if (MIXED)
             target_eval_mixed_kernel<KIND, N0, N1, N2, EVAL_FAR><<<m.n_tleaf, FAR_THREADS, 0, st>>>(ea);
         else
-            target_eval_kernel<KIND, N0, N1, N2, EVAL_FAR><<<m.n_tleaf, EVAL_THREADS, 0, st>>>(ea);
+        {
+            // without the plan; orders above (4, 7, 7) by the runtime-order sums
+            constexpr bool FIX = N0 > 0 && N0 <= 4;
+            target_eval_kernel<KIND, FIX ? N0 : 0, FIX ? N1 : 0, FIX ? N2 : 0, EVAL_FAR>
+                <<<m.n_tleaf, EVAL_THREADS, 0, st>>>(ea);
+        }
         IFGF_CHECK_LAUNCH();
         if (hk)
             hk->end();
@@ -2460,6 +2188,13 @@ int launch_mult_kernels(const MultPtrs& m, const void* d_w, void* d_u, bool real
         IFGF_RUN(3, 6, 6);
     if (lo[0] == 4 && lo[1] == 7 && lo[2] == 7)
         IFGF_RUN(4, 7, 7);
+    // p = 11 and 12 (with runtime orders the FP64 matvec at N = 3e4, p = 12
+    // took 60.7 ms: upward 36.7, far field 13.4, coarse-to-fine 7.7; fixed
+    // orders: 6.2, 0.9 and 1.0, 9.9 in all)
+    if (lo[0] == 5 && lo[1] == 8 && lo[2] == 8)
+        IFGF_RUN(5, 8, 8);
+    if (lo[0] == 6 && lo[1] == 9 && lo[2] == 9)
+        IFGF_RUN(6, 9, 9);
     IFGF_RUN(0, 0, 0);
 #undef IFGF_RUN
 }

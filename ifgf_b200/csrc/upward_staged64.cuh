@@ -82,7 +82,9 @@ __device__ __noinline__ bool ups64_fallback(const UpArgs& a, int box, int el, in
     return upward_fallback64<KIND, 0, 0, 0>(a, box, el, n, cb, fm, v);
 }
 
-constexpr int UPS64_THREADS = 64;
+// Threads: blocks of more than 200 coefficients leave room for fewer CTAs per
+// SM, so these take twice as many.
+__host__ __device__ constexpr int ups64_threads(int p_lo) { return p_lo > 200 ? 128 : 64; }
 
 // Stride (in double2) of a staged block: odd, so that the blocks of eight
 // consecutive runs start in eight different 16-byte bank groups.
@@ -103,9 +105,9 @@ template <int N0, int N1, int N2> size_t ups64_smem(int P_hi, int rch, int fe_pa
            ((size_t)16 * (fe_pad + 1) + 16) * sizeof(int);
 }
 
-// Entries evaluated together per thread (sharing every coefficient load) and
-// CTAs per SM the register budget is set for (128 registers).
-constexpr int UPS64_R = 2, UPS64_CTAS = 8;
+// Entries evaluated together per thread (sharing every coefficient load);
+// CTAs per SM give every thread 128 registers.
+constexpr int UPS64_R = 2;
 
 // One CTA per parent cone (CTAs ordered by cone element, so that consecutive
 // ones share their geometry-table rows in L2).  When it starts it resolves
@@ -124,11 +126,12 @@ constexpr int UPS64_R = 2, UPS64_CTAS = 8;
 // 4 / 64 / 16 / 4 35.6, 4 / 32 / 8 / 12 35.5: warps in flight are worth more
 // than fewer loads.
 template <int KIND, int N0, int N1, int N2>
-__global__ void __launch_bounds__(UPS64_THREADS, UPS64_CTAS)
+__global__ void __launch_bounds__(ups64_threads(N0* N1* N2), 512 / ups64_threads(N0 * N1 * N2))
     upward_staged64_kernel(const __grid_constant__ UpArgs a)
 {
     constexpr int R = UPS64_R;
     constexpr int P_LO = N0 * N1 * N2;
+    constexpr int THREADS = ups64_threads(P_LO);
     constexpr int BS = ups64_stride(P_LO);
     constexpr int SUB = UPGEO_RUN / R; // work items per table group
     constexpr bool REAL = KIND == K_LAPLACE;
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__(UPS64_THREADS, UPS64_CTAS)
     const int box = a.cc_box[c], el = a.cc_el[c];
     const int warp = threadIdx.x >> 5;
     const int ngroups = a.P_pad / UPGEO_RUN;
-    for (int n = threadIdx.x; n < a.P_hi; n += UPS64_THREADS)
+    for (int n = threadIdx.x; n < a.P_hi; n += THREADS)
         acc[n] = make_double2(0.0, 0.0);
     if (threadIdx.x < 8)
     {
@@ -154,7 +157,7 @@ __global__ void __launch_bounds__(UPS64_THREADS, UPS64_CTAS)
     __syncthreads();
     const LevelGeom& C = a.GC;
     const long long nf = (long long)C.nf[0] * C.nf[1] * C.nf[2];
-    for (int i = threadIdx.x; i < 8 * FL; i += UPS64_THREADS)
+    for (int i = threadIdx.x; i < 8 * FL; i += THREADS)
     {
         const int o = i / FL, r = i - o * FL;
         const int cb = a.T.box_child[8 * box + o];
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(UPS64_THREADS, UPS64_CTAS)
             // the next run's first group, or the row's end
             const int g_end = r1 < nrun ? rg[r1] : row_n[8 + o];
             __syncthreads(); // the previous runs' blocks are no longer read
-            for (int r = r0 + warp; r < r1; r += UPS64_THREADS / 32)
+            for (int r = r0 + warp; r < r1; r += THREADS / 32)
             {
                 const int gf = rgf[r];
                 if (gf < 0)
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(UPS64_THREADS, UPS64_CTAS)
             }
             cp_async_wait_all();
             __syncthreads();
-            for (int it = threadIdx.x; it < (g_end - g_beg) * SUB; it += UPS64_THREADS)
+            for (int it = threadIdx.x; it < (g_end - g_beg) * SUB; it += THREADS)
             {
                 const int h = it % SUB, g = g_beg + it / SUB;
                 int rl = 0; // the group's run, relative to r0
@@ -244,6 +247,6 @@ __global__ void __launch_bounds__(UPS64_THREADS, UPS64_CTAS)
         }
     }
     __syncthreads();
-    for (int n = threadIdx.x; n < a.P_hi; n += UPS64_THREADS)
+    for (int n = threadIdx.x; n < a.P_hi; n += THREADS)
         a.cvals[(size_t)c * a.P_hi + n] = acc[n];
 }
