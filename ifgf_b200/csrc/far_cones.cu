@@ -121,20 +121,70 @@ unsigned blocks_for(long long n)
 
 } // namespace
 
+namespace
+{
+
+// Places of a plan's arrays in its one allocation; the build's scratch shares
+// the values' place.
+struct Layout
+{
+    long long n_fine = 0, pairs = 0, most = 0;
+    size_t bytes = 0, scan_b = 0, count_b = 0;
+    size_t val, pos, tgt, tile, meta, host, leaf, trig, lev;
+    bool fits = false; // there are pairs, and fewer than 2^31 places
+    explicit Layout(const FarConeBuild& b)
+    {
+        size_t n_trig = 0;
+        for (const LevelGeom& G : *b.lv)
+        {
+            n_fine += G.n_fine;
+            n_trig += (size_t)(G.nf[1] + G.nf[2]);
+        }
+        pairs = b.leaf_off->back();
+        // places at most: every cone with pairs wastes less than a tile
+        most = (pairs + (FAR_TILE - 1) * std::min(n_fine, pairs) + 31) / 32 * 32;
+        fits = pairs > 0 && n_fine > 0 && most < (1ll << 31) - 1;
+        if (!fits)
+            return;
+        cub::DeviceScan::ExclusiveSum(nullptr, scan_b, (int*)nullptr, (int*)nullptr,
+                                      (int)n_fine + 1);
+        auto place = [&](size_t n) {
+            const size_t at = bytes;
+            bytes += (n + 255) / 256 * 256;
+            return at;
+        };
+        count_b = ((size_t)(n_fine + 1) * sizeof(int) + 255) / 256 * 256;
+        val = place(std::max((size_t)most * sizeof(double2), 2 * count_b + scan_b));
+        pos = place((size_t)pairs * sizeof(int));
+        tgt = place((size_t)most * sizeof(int));
+        tile = place((size_t)most / FAR_TILE * sizeof(int));
+        meta = place((size_t)n_fine * sizeof(int2));
+        host = bytes; // from here on filled on the host
+        leaf = place(b.leaf_off->size() * sizeof(long long));
+        trig = place(n_trig * sizeof(double2));
+        lev = place(b.lv->size() * sizeof(int2));
+    }
+};
+
+} // namespace
+
+void reserve_far_cones(const FarConeBuild& b, FarConePlan& plan)
+{
+    const Layout at(b);
+    if (at.fits && at.bytes <= FAR_CONES_RESERVE)
+        plan.mem.alloc(at.bytes);
+}
+
 void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
 {
     const auto start = std::chrono::steady_clock::now();
-    plan.release();
     const std::vector<LevelGeom>& lv = *b.lv;
     const int L = (int)lv.size(), nl = b.n_tleaf;
-    long long n_fine = 0;
-    for (const LevelGeom& G : lv)
-        n_fine += G.n_fine;
-    const long long pairs = b.leaf_off->back();
-    // places at most: every cone with pairs wastes less than a tile
-    const long long most =
-        (pairs + (FAR_TILE - 1) * std::min(n_fine, pairs) + 31) / 32 * 32;
-    if (pairs <= 0 || n_fine <= 0 || most >= (1ll << 31) - 1)
+    const Layout at(b);
+    const long long n_fine = at.n_fine;
+    if (plan.mem.n < at.bytes)
+        plan.mem.release();
+    if (!at.fits)
     {
         plan.refused = true;
         return;
@@ -155,30 +205,11 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
                 trig.push_back(make_double2(std::sin(c), std::cos(c)));
             }
     }
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, (int*)nullptr, (int*)nullptr, (int)n_fine + 1);
-    // one allocation; the scratch of the build shares the values' place
-    size_t used_b = 0;
-    auto place = [&](size_t bytes) {
-        const size_t at = used_b;
-        used_b += (bytes + 255) / 256 * 256;
-        return at;
-    };
-    const size_t cb = ((size_t)(n_fine + 1) * sizeof(int) + 255) / 256 * 256;
-    const size_t o_val = place(std::max((size_t)most * sizeof(double2), 2 * cb + tb));
-    const size_t o_pos = place((size_t)pairs * sizeof(int));
-    const size_t o_tgt = place((size_t)most * sizeof(int));
-    const size_t o_tile = place((size_t)most / FAR_TILE * sizeof(int));
-    const size_t o_meta = place((size_t)n_fine * sizeof(int2));
-    const size_t o_host = used_b;
-    const size_t o_leaf = place(b.leaf_off->size() * sizeof(long long));
-    const size_t o_trig = place(trig.size() * sizeof(double2));
-    const size_t o_lev = place(level.size() * sizeof(int2));
-    if (used_b > (size_t(256) << 20))
+    if (!plan.mem.p && at.bytes > (size_t(256) << 20))
     {
         size_t free_b = 0, total_b = 0;
         IFGF_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        if (used_b > free_b / 4)
+        if (at.bytes > free_b / 4)
         {
             plan.refused = true;
             return;
@@ -186,7 +217,8 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
     }
     try
     {
-        plan.mem.alloc(used_b);
+        if (!plan.mem.p)
+            plan.mem.alloc(at.bytes);
     }
     catch (const Error&)
     {
@@ -194,23 +226,24 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
         return;
     }
     unsigned char* m = plan.mem.p;
-    std::vector<unsigned char> host(used_b - o_host);
+    std::vector<unsigned char> host(at.bytes - at.host);
     std::copy_n((const unsigned char*)b.leaf_off->data(), b.leaf_off->size() * sizeof(long long),
-                host.data() + (o_leaf - o_host));
+                host.data() + (at.leaf - at.host));
     std::copy_n((const unsigned char*)trig.data(), trig.size() * sizeof(double2),
-                host.data() + (o_trig - o_host));
+                host.data() + (at.trig - at.host));
     std::copy_n((const unsigned char*)level.data(), level.size() * sizeof(int2),
-                host.data() + (o_lev - o_host));
-    IFGF_CUDA(cudaMemcpy(m + o_host, host.data(), host.size(), cudaMemcpyHostToDevice));
-    int* pos = (int*)(m + o_pos);
-    int* tgt = (int*)(m + o_tgt);
-    int* tile = (int*)(m + o_tile);
-    int2* meta = (int2*)(m + o_meta);
-    const long long* leaf_off = (const long long*)(m + o_leaf);
-    int* count = (int*)(m + o_val);
-    int* off = (int*)(m + o_val + cb);
+                host.data() + (at.lev - at.host));
+    IFGF_CUDA(cudaMemcpy(m + at.host, host.data(), host.size(), cudaMemcpyHostToDevice));
+    int* pos = (int*)(m + at.pos);
+    int* tgt = (int*)(m + at.tgt);
+    int* tile = (int*)(m + at.tile);
+    int2* meta = (int2*)(m + at.meta);
+    const long long* leaf_off = (const long long*)(m + at.leaf);
+    int* count = (int*)(m + at.val);
+    int* off = (int*)(m + at.val + at.count_b);
+    size_t scan_b = at.scan_b;
     IFGF_CUDA(cudaMemsetAsync(count, 0, (n_fine + 1) * sizeof(int), nullptr));
-    IFGF_CUDA(cudaMemsetAsync(tgt, 0xff, o_meta - o_tgt, nullptr)); // and the tiles
+    IFGF_CUDA(cudaMemsetAsync(tgt, 0xff, at.meta - at.tgt, nullptr)); // and the tiles
     for (int l = 0; l < L; l++)
         if (lv[l].n_fine > 0)
             meta_kernel<<<blocks_for(lv[l].n_fine), 256>>>(b.cone_box[l], b.cone_el[l],
@@ -219,7 +252,8 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
     count_kernel<<<nl, THREADS>>>(b.lv_dev, b.T, b.tx, b.ty, b.tz, b.fmap, b.tl_first, b.tl_last,
                                   b.far_off, b.far_src, leaf_off, pos, count, b.err);
     pad_kernel<<<blocks_for(n_fine), 256>>>(count, (int)n_fine);
-    IFGF_CUDA(cub::DeviceScan::ExclusiveSum(m + o_val + 2 * cb, tb, count, off, (int)n_fine + 1));
+    IFGF_CUDA(cub::DeviceScan::ExclusiveSum(m + at.val + 2 * at.count_b, scan_b, count, off,
+                                            (int)n_fine + 1));
     tile_kernel<<<blocks_for(n_fine), 256>>>(off, (int)n_fine, tile);
     int used = 0;
     IFGF_CUDA(cudaMemcpy(&used, off + n_fine, sizeof(int), cudaMemcpyDeviceToHost));
@@ -233,11 +267,17 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
         plan.refused = true;
         return;
     }
-    plan.pairs = pairs;
+    plan.pairs = at.pairs;
     plan.places = ((long long)used + 31) / 32 * 32;
-    plan.p = FarConePtrs{tile, plan.places / 32, tgt,      meta,
-                         (const int2*)(m + o_lev),   (const double2*)(m + o_trig),
-                         pos,  leaf_off,             (double2*)(m + o_val)};
+    plan.p = FarConePtrs{tile,
+                         plan.places / 32,
+                         tgt,
+                         meta,
+                         (const int2*)(m + at.lev),
+                         (const double2*)(m + at.trig),
+                         pos,
+                         leaf_off,
+                         (double2*)(m + at.val)};
     plan.ready = true;
     plan.ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - start)
                   .count();

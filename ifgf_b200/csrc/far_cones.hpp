@@ -41,10 +41,15 @@ struct FarConeBuild
     unsigned long long* err;
 };
 
+// A plan is one allocation.  Small ones (up to FAR_CONES_RESERVE) get it with
+// the operator's other buffers at init: an allocation of 2 MB or more takes
+// some 0.35 ms, as long as everything else a small plan's build does.
+constexpr size_t FAR_CONES_RESERVE = size_t(64) << 20;
+void reserve_far_cones(const FarConeBuild& b, FarConePlan& plan);
+
 // Fills `plan`, or leaves it empty with `refused` set: no far pairs, 2^31
-// places or more, or more than a quarter of the free device memory.  One
-// allocation: with separate ones a plan of 3e5 pairs took 1.3 ms, now 0.5
-// (3.9e8 pairs: 12 ms).  Synchronises the device.
+// places or more, or more than a quarter of the free device memory (3.9e8
+// pairs take 12 ms).  Synchronises the device.
 void build_far_cones(const FarConeBuild& b, FarConePlan& plan);
 
 } // namespace ifgf

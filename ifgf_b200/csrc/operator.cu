@@ -1102,6 +1102,38 @@ void Operator::init(const double* srcs, int64_t ns, const double* tgts, int64_t 
     init_ms_ = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// low orders with a far-cone kernel (launch_mult_kernels' fixed orders)
+static bool far_cone_shape(const int* lo)
+{
+    return lo[0] >= 2 && lo[0] <= 6 && lo[1] == lo[0] + 3 && lo[2] == lo[0] + 3;
+}
+
+static FarConeBuild far_cone_build(const DeviceState& D, const std::vector<LevelGeom>& lv)
+{
+    FarConeBuild b;
+    b.lv = &lv;
+    b.lv_dev = D.lv.p;
+    b.T = TreeArgs{D.box_c.p, D.box_H.p, D.box_first.p, D.box_last.p, D.box_child.p,
+                   D.box_level.p, D.box_leaf.p};
+    b.tx = D.tx.p;
+    b.ty = D.ty.p;
+    b.tz = D.tz.p;
+    b.fmap = D.fmap.p;
+    b.tl_first = D.tl_first.p;
+    b.tl_last = D.tl_last.p;
+    b.far_off = D.tl_far_off.p;
+    b.leaf_off = &D.tl_pair_off;
+    b.far_src = D.tl_far_src.p;
+    b.n_tleaf = D.n_tleaf;
+    for (size_t l = 0; l < lv.size(); l++)
+    {
+        b.cone_box.push_back(D.fc_box[l].p);
+        b.cone_el.push_back(D.fc_el[l].p);
+    }
+    b.err = D.err.p;
+    return b;
+}
+
 void Operator::setup_device(const double* normals)
 {
     DeviceState& D = *dev_;
@@ -1571,6 +1603,8 @@ void Operator::setup_device(const double* normals)
     D.c2f_smem = (P_hi + sz2 + (size_t)F0 * F1 * hi_[2]) * sizeof(double2);
     if (D.c2f_smem > 220 * 1024)
         throw Error(ERR_INVALID, "interpolation order too high for the coarse-to-fine kernel");
+    if (precision_ == PREC_FP64 && far_plan_on_ && far_cone_shape(lo_))
+        reserve_far_cones(far_cone_build(D, lv_), D.fc);
     phase("buffers");
 }
 
@@ -1783,7 +1817,7 @@ void Operator::set_far_plan(bool on)
 void Operator::ensure_far_cones(MultPtrs& m, void* stream)
 {
     DeviceState& D = *dev_;
-    if (!far_plan_on_ || D.n_tleaf == 0)
+    if (!far_plan_on_ || D.n_tleaf == 0 || !far_cone_shape(lo_))
         return;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess)
@@ -1795,26 +1829,7 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
     if (!D.fc.ready && !D.fc.refused && !capturing)
     {
         IFGF_CUDA(cudaSetDevice(device_));
-        FarConeBuild b;
-        b.lv = &lv_;
-        b.lv_dev = D.lv.p;
-        b.T = m.T;
-        b.tx = D.tx.p;
-        b.ty = D.ty.p;
-        b.tz = D.tz.p;
-        b.fmap = D.fmap.p;
-        b.tl_first = D.tl_first.p;
-        b.tl_last = D.tl_last.p;
-        b.far_off = D.tl_far_off.p;
-        b.leaf_off = &D.tl_pair_off;
-        b.far_src = D.tl_far_src.p;
-        b.n_tleaf = D.n_tleaf;
-        for (size_t l = 0; l < lv_.size(); l++)
-        {
-            b.cone_box.push_back(D.fc_box[l].p);
-            b.cone_el.push_back(D.fc_el[l].p);
-        }
-        b.err = D.err.p;
+        const FarConeBuild b = far_cone_build(D, lv_);
         build_far_cones(b, D.fc);
     }
     if (!D.fc.ready)
