@@ -625,22 +625,172 @@ constexpr int EVAL_THREADS = 128;
 constexpr int FAR_THREADS = 256;
 constexpr int EVAL_NEAR = 0, EVAL_FAR = 1; // the two passes of target evaluation
 
-// One CTA per target leaf.  A leaf holds fewer targets than threads, so
-// thread (ti, si) takes target ti and every S-th near source / far box
-// (S = threads / targets); the S partial sums are added in a fixed order.
-template <int KIND, int N0, int N1, int N2, int PART>
+// Near field: one CTA per target leaf.  The leaf's near source boxes hold a
+// few dozen points each, so their ranges are scanned into one sequence and the
+// CTA stages 256 sources of it at a time, the next ones loading while it
+// evaluates; thread (ti, si) takes target ti and every S-th staged source
+// (S = threads / targets), two at a time; the S partial sums are added in a
+// fixed order.  Bound by the FP64 pipe.  Per matvec 6.2 ms at N = 1e6, 1.3 at
+// 2e5, 0.09 at 2e4 (Laplace); staging one box at a time with 128 threads and
+// two barriers a box took 8.5, 2.0 and 0.25 (10.7, 2.6 and 0.40 with the
+// library functions).
+constexpr int NEAR_THREADS = 256;
+template <int KIND>
+__global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_constant__ EvalArgs a)
+{
+    using P = Plugin<KIND>;
+    constexpr int TH = NEAR_THREADS;
+    // per source (x, y), (z, Re w), (Im w, n0), (n1, n2)
+    constexpr int ROWS = P::needs_normals ? 4 : 3;
+    __shared__ __align__(16) double2 src[ROWS * TH];
+    __shared__ double2 part[TH];
+    __shared__ int pre[TH + 1], first[TH], wsum[TH / 32];
+    const int tl = blockIdx.x, tid = threadIdx.x;
+    const int tf = a.tl_first[tl], tlast = a.tl_last[tl];
+    const long long nb0 = a.near_off[tl], nb1 = a.near_off[tl + 1];
+    const KParamsRegs kp(a.kp);
+    for (int base = tf; base < tlast; base += TH)
+    {
+        const int cnt = min(TH, tlast - base);
+        const int S = TH / cnt;
+        const int ti = tid % cnt, si = tid / cnt;
+        const bool active = si < S;
+        const int t = base + ti;
+        const double y0 = a.tx[t], y1 = a.ty[t], y2 = a.tz[t];
+        cplx<double> acc = {0.0, 0.0};
+        for (long long b0 = nb0; b0 < nb1; b0 += TH)
+        {
+            // prefix sums of the sources in up to TH boxes
+            const int nb = (int)min((long long)TH, nb1 - b0);
+            int n = 0, f = 0;
+            if (tid < nb)
+            {
+                const int sb = a.near_src[b0 + tid];
+                f = a.T.box_first[sb];
+                n = a.T.box_last[sb] - f;
+            }
+            int sum = n;
+#pragma unroll
+            for (int m = 1; m < 32; m <<= 1)
+            {
+                const int o = __shfl_up_sync(~0u, sum, m);
+                if ((tid & 31) >= m)
+                    sum += o;
+            }
+            __syncthreads(); // the previous boxes' tables are no longer read
+            if ((tid & 31) == 31)
+                wsum[tid >> 5] = sum;
+            __syncthreads();
+            for (int w = 0; w < (tid >> 5); w++)
+                sum += wsum[w];
+            pre[tid + 1] = sum;
+            first[tid] = f;
+            if (tid == 0)
+                pre[0] = 0;
+            __syncthreads();
+            const int total = pre[nb];
+            double2 v0, v1, v2, v3;
+            auto fetch = [&](int c) {
+                const int q = c + tid;
+                if (q >= total)
+                    return;
+                int lo = 0, hi = nb; // pre[lo] <= q < pre[hi]
+                while (hi - lo > 1)
+                {
+                    const int mid = (lo + hi) >> 1;
+                    if (pre[mid] <= q)
+                        lo = mid;
+                    else
+                        hi = mid;
+                }
+                const int i = first[lo] + (q - pre[lo]);
+                const double2 wv = a.w[i];
+                v0 = make_double2(a.S.sx[i], a.S.sy[i]);
+                v1 = make_double2(a.S.sz[i], wv.x);
+                v2 = make_double2(wv.y, P::needs_normals ? a.S.nx[i] : 0.0);
+                if (P::needs_normals)
+                    v3 = make_double2(a.S.ny[i], a.S.nz[i]);
+            };
+            fetch(0);
+            for (int c = 0; c < total; c += TH)
+            {
+                const int ccnt = min(TH, total - c);
+                __syncthreads(); // the previous chunk is no longer read
+                if (tid < ccnt)
+                {
+                    double2* s = src + ROWS * tid;
+                    s[0] = v0;
+                    s[1] = v1;
+                    s[2] = v2;
+                    if (P::needs_normals)
+                        s[ROWS - 1] = v3;
+                }
+                __syncthreads();
+                fetch(c + TH);
+                if (!active)
+                    continue;
+                for (int i = si; i < ccnt; i += 2 * S)
+                {
+                    const bool two = i + S < ccnt;
+                    double x[2][3], nv[2][3];
+                    cplx<double> w[2];
+                    bool tiny = false;
+#pragma unroll
+                    for (int r = 0; r < 2; r++)
+                    {
+                        const double2* s = src + ROWS * (r == 0 || !two ? i : i + S);
+                        const double2 s0 = s[0], s1 = s[1], s2 = s[2];
+                        const double2 s3 = P::needs_normals ? s[ROWS - 1] : make_double2(0.0, 0.0);
+                        x[r][0] = s0.x - y0;
+                        x[r][1] = s0.y - y1;
+                        x[r][2] = s1.x - y2;
+                        w[r] = {s1.y, s2.x};
+                        nv[r][0] = s2.y, nv[r][1] = s3.x, nv[r][2] = s3.y;
+                        tiny |= tiny_square(dot3(x[r], x[r]));
+                    }
+                    if (!two)
+                        w[1] = {0.0, 0.0};
+                    if (!tiny)
+                    {
+#pragma unroll
+                        for (int r = 0; r < 2; r++)
+                            cfma(acc, w[r], P::kernel4pi(x[r], nv[r], kp));
+                    }
+                    else
+#pragma unroll
+                        for (int r = 0; r < 2; r++)
+                            cfma(acc, w[r], P::kernel4pi(x[r], nv[r], a.kp));
+                }
+            }
+        }
+        __syncthreads();
+        part[tid] = make_double2(acc.re, acc.im);
+        __syncthreads();
+        if (si == 0)
+        {
+            double sr = 0, sim = 0;
+            for (int s = 0; s < S; s++)
+            {
+                sr += part[ti + s * cnt].x;
+                sim += part[ti + s * cnt].y;
+            }
+            a.unear[t] = make_double2(INV4PI * sr, INV4PI * sim);
+        }
+    }
+}
+
+// Far field without the far-cone plan: one CTA per target leaf.  A leaf holds
+// fewer targets than threads, so thread (ti, si) takes target ti and every
+// S-th far box (S = threads / targets); the S partial sums are added in a
+// fixed order, then the near sum.
+template <int KIND, int N0, int N1, int N2>
 __global__ void __launch_bounds__(EVAL_THREADS) target_eval_kernel(EvalArgs a)
 {
     using P = Plugin<KIND>;
-    __shared__ double xs[EVAL_THREADS], ys[EVAL_THREADS], zs[EVAL_THREADS];
-    __shared__ double wr[EVAL_THREADS], wi[EVAL_THREADS];
-    __shared__ double n0[P::needs_normals ? EVAL_THREADS : 1], n1[P::needs_normals ? EVAL_THREADS : 1],
-        n2[P::needs_normals ? EVAL_THREADS : 1];
     __shared__ double rr[EVAL_THREADS], ri[EVAL_THREADS];
     const int tl = blockIdx.x;
     const int tf = a.tl_first[tl], tlast = a.tl_last[tl];
-    const long long nb0 = a.near_off[tl], nb1 = PART == EVAL_NEAR ? a.near_off[tl + 1] : nb0;
-    const long long fb0 = a.far_off[tl], fb1 = PART == EVAL_FAR ? a.far_off[tl + 1] : fb0;
+    const long long fb0 = a.far_off[tl], fb1 = a.far_off[tl + 1];
     for (int base = tf; base < tlast; base += EVAL_THREADS)
     {
         const int cnt = min(EVAL_THREADS, tlast - base);
@@ -650,42 +800,6 @@ __global__ void __launch_bounds__(EVAL_THREADS) target_eval_kernel(EvalArgs a)
         const int t = base + ti;
         const double y0 = a.tx[t], y1 = a.ty[t], y2 = a.tz[t];
         cplx<double> acc = {0.0, 0.0};
-        for (long long e = nb0; e < nb1; e++)
-        {
-            const int sb = a.near_src[e];
-            const int sf = a.T.box_first[sb], sl = a.T.box_last[sb];
-            for (int cs = sf; cs < sl; cs += EVAL_THREADS)
-            {
-                const int ccnt = min(EVAL_THREADS, sl - cs);
-                __syncthreads();
-                if (threadIdx.x < ccnt)
-                {
-                    const int i = cs + threadIdx.x;
-                    xs[threadIdx.x] = a.S.sx[i];
-                    ys[threadIdx.x] = a.S.sy[i];
-                    zs[threadIdx.x] = a.S.sz[i];
-                    const double2 wv = a.w[i];
-                    wr[threadIdx.x] = wv.x;
-                    wi[threadIdx.x] = wv.y;
-                    if (P::needs_normals)
-                    {
-                        n0[threadIdx.x] = a.S.nx[i];
-                        n1[threadIdx.x] = a.S.ny[i];
-                        n2[threadIdx.x] = a.S.nz[i];
-                    }
-                }
-                __syncthreads();
-                if (active)
-                    for (int i = si; i < ccnt; i += S)
-                    {
-                        const double x[3] = {xs[i] - y0, ys[i] - y1, zs[i] - y2};
-                        const double nv[3] = {P::needs_normals ? n0[i] : 0.0,
-                                              P::needs_normals ? n1[i] : 0.0,
-                                              P::needs_normals ? n2[i] : 0.0};
-                        cfma(acc, cplx<double>{wr[i], wi[i]}, P::kernel4pi(x, nv, a.kp));
-                    }
-            }
-        }
         if (active)
             for (long long e = fb0 + si; e < fb1; e += S)
             {
@@ -721,21 +835,16 @@ __global__ void __launch_bounds__(EVAL_THREADS) target_eval_kernel(EvalArgs a)
                 sr += rr[ti + s * cnt];
                 sim += ri[ti + s * cnt];
             }
-            if (PART == EVAL_NEAR)
-                a.unear[t] = make_double2(INV4PI * sr, INV4PI * sim);
+            const double2 nr = a.unear[t];
+            sr += nr.x;
+            sim += nr.y;
+            const long long o = a.tgt_perm[t];
+            if (a.real_out)
+                a.out[o] = sr;
             else
             {
-                const double2 nr = a.unear[t];
-                sr += nr.x;
-                sim += nr.y;
-                const long long o = a.tgt_perm[t];
-                if (a.real_out)
-                    a.out[o] = sr;
-                else
-                {
-                    a.out[2 * o] = sr;
-                    a.out[2 * o + 1] = sim;
-                }
+                a.out[2 * o] = sr;
+                a.out[2 * o + 1] = sim;
             }
         }
     }
@@ -1983,7 +2092,7 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         if (MIXED)
             target_eval_mixed_kernel<KIND, 0, 0, 0, EVAL_NEAR><<<m.n_tleaf, EVAL_THREADS, 0, ns>>>(ea);
         else
-            target_eval_kernel<KIND, 0, 0, 0, EVAL_NEAR><<<m.n_tleaf, EVAL_THREADS, 0, ns>>>(ea);
+            near_kernel<KIND><<<m.n_tleaf, NEAR_THREADS, 0, ns>>>(ea);
         IFGF_CHECK_LAUNCH();
         if (hk)
             hk->end();
@@ -2163,7 +2272,7 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         {
             // without the plan; orders above (4, 7, 7) by the runtime-order sums
             constexpr bool FIX = N0 > 0 && N0 <= 4;
-            target_eval_kernel<KIND, FIX ? N0 : 0, FIX ? N1 : 0, FIX ? N2 : 0, EVAL_FAR>
+            target_eval_kernel<KIND, FIX ? N0 : 0, FIX ? N1 : 0, FIX ? N2 : 0>
                 <<<m.n_tleaf, EVAL_THREADS, 0, st>>>(ea);
         }
         IFGF_CHECK_LAUNCH();
