@@ -1468,6 +1468,17 @@ void Operator::setup_device(const double* normals)
             std::vector<int> el(lv_[l].n_coarse);
             IFGF_CUDA(cudaMemcpy(el.data(), D.cc_el[l].p, el.size() * sizeof(int),
                                  cudaMemcpyDeviceToHost));
+            // within an element by the children the boxes have (about half of
+            // the eight on a surface): the row tiles of the tensor-core kernels
+            // take consecutive cones of an element and skip the octants where
+            // none of them has a child
+            std::vector<int> cbox(lv_[l].n_coarse), mask(lv_[l].n_coarse, 0);
+            IFGF_CUDA(cudaMemcpy(cbox.data(), D.cc_box[l].p, cbox.size() * sizeof(int),
+                                 cudaMemcpyDeviceToHost));
+            for (int i : uidx)
+                for (int o = 0; o < 8; o++)
+                    mask[i] |= (bch[8 * cbox[i] + o] >= 0) << o;
+            stable_order_by_key(uidx, mask);
             stable_order_by_key(uidx, el);
             for (size_t i = 0; i < uidx.size(); i++)
             {
@@ -1512,9 +1523,6 @@ void Operator::setup_device(const double* normals)
                 UpwardLevelStats& us = up_stats_[l];
                 us.cones = (int64_t)uidx.size();
                 us.slots = ns;
-                std::vector<int> cbox(lv_[l].n_coarse);
-                IFGF_CUDA(cudaMemcpy(cbox.data(), D.cc_box[l].p, cbox.size() * sizeof(int),
-                                     cudaMemcpyDeviceToHost));
                 for (size_t i = 0; i < uidx.size(); i++)
                 {
                     const int g = cbox[uidx[i]];
