@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(FARB_THREADS, FARB_CTAS)
                 const double2 nr = bp.unear[(size_t)(pb + r) * bp.n_tgt + t];
                 sr += nr.x;
                 sim += nr.y;
-                double* out = a.out + (size_t)(pb + r) * bp.out_plane;
+                double* out = a.out + (size_t)(bp.row ? bp.row[pb + r] : pb + r) * bp.out_plane;
                 if (a.real_out)
                     out[o] = sr;
                 else
@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(FARB_THREADS, far_plan_ctas(NSL, N0 * N1 * N2,
             const double2 nr = bp.unear[(size_t)(pb + r) * bp.n_tgt + t];
             sr += nr.x;
             sim += nr.y;
-            double* out = a.out + (size_t)(pb + r) * bp.out_plane;
+            double* out = a.out + (size_t)(bp.row ? bp.row[pb + r] : pb + r) * bp.out_plane;
             if (a.real_out)
                 out[o] = sr;
             else

@@ -320,6 +320,12 @@ struct BatchPtrs
     // the distance tables (UpGeo32::tr = d - d_parent, ::ti = d_parent / d)
     const KParams* kp_plane = nullptr;
     const UpGeo32* const* dgeo32 = nullptr; // per level (host array)
+    // with kp_plane: the caller's row of every plane (in_plane / out_plane
+    // strides from the whole call's buffers), and whether an odd plane's
+    // wavenumber is the complex conjugate of the plane before it, whose
+    // kernel values are then the conjugates
+    const int* row = nullptr;
+    const int* conj_prev = nullptr;
     // tensor-core upward tiles for groups * BATCH_NB planes, per level (host
     // arrays; null: FFMA kernel)
     const int4* const* tc_tiles = nullptr;

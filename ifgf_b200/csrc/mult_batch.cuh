@@ -18,7 +18,8 @@
 // Permuted FP32 densities of nrhs right-hand sides; planes past nrhs zero.
 static __global__ void permute_batch_kernel(const double* __restrict__ in, int real_in,
                                             const long long* __restrict__ perm, float2* w,
-                                            long long n, int nrhs, long long in_plane)
+                                            long long n, int nrhs, long long in_plane,
+                                            const int* __restrict__ row)
 {
     const int b = blockIdx.y;
     float2* wb = w + (size_t)b * n;
@@ -31,7 +32,7 @@ static __global__ void permute_batch_kernel(const double* __restrict__ in, int r
             continue;
         }
         const long long j = perm[i];
-        const double* src = in + (size_t)b * in_plane;
+        const double* src = in + (size_t)(row ? row[b] : b) * in_plane;
         if (real_in)
             wb[i] = make_float2((float)src[j], 0.f);
         else
@@ -53,7 +54,9 @@ static __global__ void permute_batch_kernel(const double* __restrict__ in, int r
 constexpr int LEAF_NPT = 4;
 // with MK every (node, plane) pair has its own kernel evaluation, so more
 // nodes per thread save no evaluations: two, at fewer registers (the
-// 64-wavenumber CQ batch at N = 1e5: 61.8 ms, 66.6 with four)
+// 64-wavenumber CQ batch at N = 1e5: 61.6 ms, 66.6 with four; 51.3 since the
+// planes of a conjugate pair share their evaluations, here (23.8 -> 17.5 ms)
+// and in the near field (12.7 -> 9.0))
 __host__ __device__ constexpr int leaf_npt(bool mk) { return mk ? 2 : LEAF_NPT; }
 inline int leaf_batch_threads(int P_hi, int npt)
 {
@@ -82,9 +85,15 @@ __global__ void __launch_bounds__(NODE_THREADS) leaf_sample_batch_kernel(LeafArg
     extern __shared__ __align__(16) float4 leaf_sm4[];
     __shared__ KParams kps[MK ? NB : 1];
     const int pb = blockIdx.z * NB; // first plane of the group
+    bool pair[NB / 2]; // planes 2 h and 2 h + 1 at conjugate wavenumbers
     if constexpr (MK)
+    {
         if (threadIdx.x < NB)
             kps[threadIdx.x] = bp.kp_plane[pb + threadIdx.x]; // read after the chunk barriers
+#pragma unroll
+        for (int h = 0; h < NB / 2; h++)
+            pair[h] = bp.conj_prev && bp.conj_prev[pb + 2 * h + 1];
+    }
     const int c = a.idx[blockIdx.x];
     const int node0 = blockIdx.y * NPQ * blockDim.x;
     const int box = a.cc_box[c], el = a.cc_el[c];
@@ -171,11 +180,14 @@ __global__ void __launch_bounds__(NODE_THREADS) leaf_sample_batch_kernel(LeafArg
                     continue;
                 if constexpr (MK)
                 {
+                    cplx<float> v = {0.f, 0.f};
 #pragma unroll
                     for (int r = 0; r < NB; r++)
                     {
-                        const cplx<float> v =
-                            P::factored(av, aai, b[q], nv, {1.f, 0.f}, dc[q], kps[r]);
+                        if (r % 2 == 1 && pair[r / 2])
+                            v.im = -v.im;
+                        else
+                            v = P::factored(av, aai, b[q], nv, {1.f, 0.f}, dc[q], kps[r]);
                         acc[q][r].re = fmaf(wr[r].x, v.re, fmaf(-wr[r].y, v.im, acc[q][r].re));
                         acc[q][r].im = fmaf(wr[r].x, v.im, fmaf(wr[r].y, v.re, acc[q][r].im));
                     }
@@ -216,9 +228,15 @@ __global__ void __launch_bounds__(EVAL_THREADS) near_batch_kernel(EvalArgs a, Ba
     constexpr int NB = BATCH_NB;
     __shared__ KParams kps[MK ? NB : 1];
     const int pb = blockIdx.y * NB;
+    bool pair[NB / 2]; // planes 2 h and 2 h + 1 at conjugate wavenumbers
     if constexpr (MK)
+    {
         if (threadIdx.x < NB)
             kps[threadIdx.x] = bp.kp_plane[pb + threadIdx.x]; // read after the chunk barriers
+#pragma unroll
+        for (int h = 0; h < NB / 2; h++)
+            pair[h] = bp.conj_prev && bp.conj_prev[pb + 2 * h + 1];
+    }
     using CT = typename std::conditional<P::needs_normals, double, float>::type;
     __shared__ CT xs[EVAL_THREADS], ys[EVAL_THREADS], zs[EVAL_THREADS];
     __shared__ float2 ws[NB][EVAL_THREADS];
@@ -283,10 +301,16 @@ __global__ void __launch_bounds__(EVAL_THREADS) near_batch_kernel(EvalArgs a, Ba
                         const double nv[3] = {n0[i], n1[i], n2[i]};
                         if constexpr (MK)
                         {
+                            cplx<float> kv = {0.f, 0.f};
 #pragma unroll
                             for (int r = 0; r < NB; r++)
-                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y},
-                                      P::kernel_d(x, nv, kps[r]));
+                            {
+                                if (r % 2 == 1 && pair[r / 2])
+                                    kv.im = -kv.im;
+                                else
+                                    kv = P::kernel_d(x, nv, kps[r]);
+                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y}, kv);
+                            }
                         }
                         else
                         {
@@ -301,10 +325,16 @@ __global__ void __launch_bounds__(EVAL_THREADS) near_batch_kernel(EvalArgs a, Ba
                         const float x[3] = {xs[i] - yl0, ys[i] - yl1, zs[i] - yl2};
                         if constexpr (MK)
                         {
+                            cplx<float> kv = {0.f, 0.f};
 #pragma unroll
                             for (int r = 0; r < NB; r++)
-                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y},
-                                      P::kernel(x, nullptr, kps[r]));
+                            {
+                                if (r % 2 == 1 && pair[r / 2])
+                                    kv.im = -kv.im;
+                                else
+                                    kv = P::kernel(x, nullptr, kps[r]);
+                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y}, kv);
+                            }
                         }
                         else
                         {
@@ -381,7 +411,8 @@ static int run_mult_batch(const MultPtrs& m, const BatchPtrs& bp, const void* d_
             if (hk)
                 hk->begin(PROF_PERMUTE);
             permute_batch_kernel<<<dim3(blocks, bp.groups * BATCH_NB), thr, 0, st>>>(
-                (const double*)d_w, real ? 1 : 0, m.src_perm, bp.w, m.n_src, bp.nrhs, bp.in_plane);
+                (const double*)d_w, real ? 1 : 0, m.src_perm, bp.w, m.n_src, bp.nrhs, bp.in_plane,
+                bp.row);
             IFGF_CHECK_LAUNCH();
             if (hk)
                 hk->end();

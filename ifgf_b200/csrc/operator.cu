@@ -88,6 +88,10 @@ struct DeviceState
     // distance tables (built on first use after an init)
     DevBuf<KParams> kp_plane;
     std::vector<KParams> kp_host; // what kp_plane holds
+    // per plane: the caller's row, then (from kp_host.size() on) whether it is
+    // the conjugate of the plane before it
+    DevBuf<int> kp_row;
+    std::vector<int> kp_row_host;
     std::vector<DevBuf<UpGeo32>> dgeo32;
     std::vector<const UpGeo32*> dgeo32_ptr;
     bool dgeo_ready = false;
@@ -2653,6 +2657,48 @@ void Operator::mult_wavenumbers_host(const double* k, int64_t nk, const void* w,
     check_device_status();
 }
 
+// Order of the wavenumbers k (re, im): pairs of complex conjugates (to a few
+// roundings; real ones pair with equal ones) first and side by side, then the
+// others; returns how many are in pairs.
+static size_t conjugate_pairs(const double* k, int64_t nk, std::vector<int64_t>& order)
+{
+    auto tol = [&](int64_t p) {
+        return 4 * 2.220446049250313e-16 * std::hypot(k[2 * p], k[2 * p + 1]);
+    };
+    std::vector<int64_t> by_re((size_t)nk);
+    for (int64_t p = 0; p < nk; p++)
+        by_re[(size_t)p] = p;
+    std::sort(by_re.begin(), by_re.end(), [&](int64_t a, int64_t b) {
+        return k[2 * a] != k[2 * b] ? k[2 * a] < k[2 * b] : a < b;
+    });
+    std::vector<char> used((size_t)nk, 0);
+    std::vector<int64_t> single;
+    for (int64_t p = 0; p < nk; p++)
+    {
+        if (used[(size_t)p])
+            continue;
+        used[(size_t)p] = 1;
+        const double t = tol(p);
+        int64_t mate = -1;
+        for (auto it = std::lower_bound(by_re.begin(), by_re.end(), k[2 * p] - t,
+                                        [&](int64_t a, double v) { return k[2 * a] < v; });
+             it != by_re.end() && k[2 * *it] <= k[2 * p] + t && mate < 0; ++it)
+            if (!used[(size_t)*it] && std::abs(k[2 * *it + 1] + k[2 * p + 1]) <= t)
+                mate = *it;
+        if (mate < 0)
+        {
+            single.push_back(p);
+            continue;
+        }
+        used[(size_t)mate] = 1;
+        order.push_back(p);
+        order.push_back(mate);
+    }
+    const size_t paired = order.size();
+    order.insert(order.end(), single.begin(), single.end());
+    return paired;
+}
+
 void Operator::mult_wavenumbers_device(const double* k, int64_t nk, const void* d_w, void* d_u,
                                        void* stream)
 {
@@ -2694,18 +2740,38 @@ void Operator::mult_wavenumbers_device(const double* k, int64_t nk, const void* 
     }
     ensure_distance_tables();
     const int planes = ensure_batch_planes(nk);
-    // every plane's wavenumber, padded to whole groups
+    // every plane's row of the call and wavenumber, padded to whole groups:
+    // conjugate pairs first, side by side, so that the kernels evaluated per
+    // wavenumber do it once for both (a convolution-quadrature set consists of
+    // such pairs; for the kernels of e^{-k r} only, whose values then are
+    // conjugates).  Wavenumbers within a few roundings count as conjugate: the
+    // mixed pipeline holds them in 48 bits.
     const int64_t nk_pad = (nk + BATCH_NB - 1) / BATCH_NB * BATCH_NB;
     std::vector<KParams> kps((size_t)nk_pad);
-    for (int64_t p = 0; p < nk_pad; p++)
+    std::vector<int> rows((size_t)(2 * nk_pad), 0);
     {
-        const int64_t q = std::min(p, nk - 1);
-        kps[(size_t)p] = make_kparams(k[2 * q], k[2 * q + 1], dx_);
+        std::vector<int64_t> order;
+        size_t paired = 0;
+        if (kind_ == K_MODHELMHOLTZ || kind_ == K_GRADHELMHOLTZ || kind_ == K_DOUBLELAYER)
+        {
+            paired = conjugate_pairs(k, nk, order);
+            for (size_t p = 1; p < paired; p += 2)
+                rows[(size_t)nk_pad + p] = 1;
+        }
+        else
+            for (int64_t p = 0; p < nk; p++)
+                order.push_back(p);
+        for (int64_t p = 0; p < nk_pad; p++)
+        {
+            const int64_t q = order[(size_t)std::min(p, nk - 1)];
+            rows[(size_t)p] = (int)q;
+            kps[(size_t)p] = make_kparams(k[2 * q], k[2 * q + 1], dx_);
+        }
     }
     // uploaded only when they change: a repeated call (the same frequency
     // set) then enqueues kernels only, so that it can be captured into a
     // CUDA graph after a first call
-    bool same_k = D.kp_host.size() == kps.size();
+    bool same_k = D.kp_host.size() == kps.size() && D.kp_row_host == rows;
     for (size_t i = 0; same_k && i < kps.size(); i++)
         same_k = D.kp_host[i].kr == kps[i].kr && D.kp_host[i].ki == kps[i].ki &&
                  D.kp_host[i].dx == kps[i].dx;
@@ -2713,10 +2779,15 @@ void Operator::mult_wavenumbers_device(const double* k, int64_t nk, const void* 
     {
         if (D.kp_plane.n < kps.size())
             D.kp_plane.alloc(kps.size());
+        if (D.kp_row.n < rows.size())
+            D.kp_row.alloc(rows.size());
         IFGF_CUDA(cudaMemcpyAsync(D.kp_plane.p, kps.data(), kps.size() * sizeof(KParams),
                                   cudaMemcpyHostToDevice, st));
-        IFGF_CUDA(cudaStreamSynchronize(st)); // kps is a temporary
+        IFGF_CUDA(cudaMemcpyAsync(D.kp_row.p, rows.data(), rows.size() * sizeof(int),
+                                  cudaMemcpyHostToDevice, st));
+        IFGF_CUDA(cudaStreamSynchronize(st)); // kps and rows are temporaries
         D.kp_host = kps;
+        D.kp_row_host = rows;
     }
     BatchPtrs bp = batch_ptrs(in_plane, out_plane);
     bp.dgeo32 = D.dgeo32_ptr.data();
@@ -2729,12 +2800,12 @@ void Operator::mult_wavenumbers_device(const double* k, int64_t nk, const void* 
         bp.nrhs = (int)std::min<int64_t>(planes, nk - done);
         bp.groups = (bp.nrhs + BATCH_NB - 1) / BATCH_NB;
         bp.kp_plane = D.kp_plane.p + done;
+        bp.row = D.kp_row.p + done;
+        bp.conj_prev = D.kp_row.p + nk_pad + done;
         EventHooks log(D, st);
         int r = -1;
-        IFGF_DISPATCH(kind_, r = launch_mult_batch_kernels<KK>(
-                                 m, bp, (const double*)d_w + done * in_plane,
-                                 (double*)d_u + done * out_plane, is_real(), st,
-                                 profiling_ ? &log : nullptr));
+        IFGF_DISPATCH(kind_, r = launch_mult_batch_kernels<KK>(m, bp, d_w, d_u, is_real(), st,
+                                                               profiling_ ? &log : nullptr));
         if (r < 0)
             throw Error(ERR_INVALID, "multi-wavenumber batches need one of the batched order "
                                      "shapes (low orders (2,5,5), (3,6,6) or (4,7,7))");
