@@ -56,7 +56,7 @@ constexpr int LEAF_NPT = 4;
 // nodes per thread save no evaluations: two, at fewer registers (the
 // 64-wavenumber CQ batch at N = 1e5: 61.6 ms, 66.6 with four; 51.3 since the
 // planes of a conjugate pair share their evaluations, here (23.8 -> 17.5 ms)
-// and in the near field (12.7 -> 9.0))
+// and in the near field (12.7 -> 9.0 ms))
 __host__ __device__ constexpr int leaf_npt(bool mk) { return mk ? 2 : LEAF_NPT; }
 inline int leaf_batch_threads(int P_hi, int npt)
 {
@@ -217,167 +217,6 @@ __global__ void __launch_bounds__(NODE_THREADS) leaf_sample_batch_kernel(LeafArg
     }
 }
 
-// Near field of a plane group (blockIdx.y): one kernel value per (target,
-// source) pair, applied to every plane (with MK one per plane); FP32 per
-// source chunk, FP64 across chunks and threads, written to the near-sum
-// planes.
-template <int KIND, bool MK>
-__global__ void __launch_bounds__(EVAL_THREADS) near_batch_kernel(EvalArgs a, BatchPtrs bp)
-{
-    using P = PluginF<KIND>;
-    constexpr int NB = BATCH_NB;
-    __shared__ KParams kps[MK ? NB : 1];
-    const int pb = blockIdx.y * NB;
-    bool pair[NB / 2]; // planes 2 h and 2 h + 1 at conjugate wavenumbers
-    if constexpr (MK)
-    {
-        if (threadIdx.x < NB)
-            kps[threadIdx.x] = bp.kp_plane[pb + threadIdx.x]; // read after the chunk barriers
-#pragma unroll
-        for (int h = 0; h < NB / 2; h++)
-            pair[h] = bp.conj_prev && bp.conj_prev[pb + 2 * h + 1];
-    }
-    using CT = typename std::conditional<P::needs_normals, double, float>::type;
-    __shared__ CT xs[EVAL_THREADS], ys[EVAL_THREADS], zs[EVAL_THREADS];
-    __shared__ float2 ws[NB][EVAL_THREADS];
-    __shared__ double n0[P::needs_normals ? EVAL_THREADS : 1], n1[P::needs_normals ? EVAL_THREADS : 1],
-        n2[P::needs_normals ? EVAL_THREADS : 1];
-    __shared__ double rr[NB][EVAL_THREADS], ri[NB][EVAL_THREADS];
-    const long long nsrc = bp.n_src;
-    const int tl = blockIdx.x;
-    const int tf = a.tl_first[tl], tlast = a.tl_last[tl];
-    const double r0 = a.tx[tf], r1 = a.ty[tf], r2 = a.tz[tf];
-    const long long nb0 = a.near_off[tl], nb1 = a.near_off[tl + 1];
-    for (int base = tf; base < tlast; base += EVAL_THREADS)
-    {
-        const int cnt = min(EVAL_THREADS, tlast - base);
-        const int S = EVAL_THREADS / cnt;
-        const int ti = threadIdx.x % cnt, si = threadIdx.x / cnt;
-        const bool active = si < S;
-        const int t = base + ti;
-        const double y0 = a.tx[t], y1 = a.ty[t], y2 = a.tz[t];
-        const float yl0 = (float)(y0 - r0), yl1 = (float)(y1 - r1), yl2 = (float)(y2 - r2);
-        double accr[NB], acci[NB];
-#pragma unroll
-        for (int r = 0; r < NB; r++)
-            accr[r] = acci[r] = 0.0;
-        for (long long e = nb0; e < nb1; e++)
-        {
-            const int sb = a.near_src[e];
-            const int sf = a.T.box_first[sb], sl = a.T.box_last[sb];
-            for (int cs = sf; cs < sl; cs += EVAL_THREADS)
-            {
-                const int ccnt = min(EVAL_THREADS, sl - cs);
-                __syncthreads();
-                if (threadIdx.x < ccnt)
-                {
-                    const int i = cs + threadIdx.x;
-                    xs[threadIdx.x] = (CT)(a.S.sx[i] - r0);
-                    ys[threadIdx.x] = (CT)(a.S.sy[i] - r1);
-                    zs[threadIdx.x] = (CT)(a.S.sz[i] - r2);
-#pragma unroll
-                    for (int r = 0; r < NB; r++)
-                        ws[r][threadIdx.x] = bp.w[(size_t)(pb + r) * nsrc + i];
-                    if (P::needs_normals)
-                    {
-                        n0[threadIdx.x] = a.S.nx[i];
-                        n1[threadIdx.x] = a.S.ny[i];
-                        n2[threadIdx.x] = a.S.nz[i];
-                    }
-                }
-                __syncthreads();
-                if (!active)
-                    continue;
-                cplx<float> acc[NB];
-#pragma unroll
-                for (int r = 0; r < NB; r++)
-                    acc[r] = {0.f, 0.f};
-                for (int i = si; i < ccnt; i += S)
-                {
-                    if constexpr (P::needs_normals)
-                    {
-                        const double yd0 = y0 - r0, yd1 = y1 - r1, yd2 = y2 - r2;
-                        const double x[3] = {xs[i] - yd0, ys[i] - yd1, zs[i] - yd2};
-                        const double nv[3] = {n0[i], n1[i], n2[i]};
-                        if constexpr (MK)
-                        {
-                            cplx<float> kv = {0.f, 0.f};
-#pragma unroll
-                            for (int r = 0; r < NB; r++)
-                            {
-                                if (r % 2 == 1 && pair[r / 2])
-                                    kv.im = -kv.im;
-                                else
-                                    kv = P::kernel_d(x, nv, kps[r]);
-                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y}, kv);
-                            }
-                        }
-                        else
-                        {
-                            const cplx<float> kv = P::kernel_d(x, nv, a.kp);
-#pragma unroll
-                            for (int r = 0; r < NB; r++)
-                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y}, kv);
-                        }
-                    }
-                    else
-                    {
-                        const float x[3] = {xs[i] - yl0, ys[i] - yl1, zs[i] - yl2};
-                        if constexpr (MK)
-                        {
-                            cplx<float> kv = {0.f, 0.f};
-#pragma unroll
-                            for (int r = 0; r < NB; r++)
-                            {
-                                if (r % 2 == 1 && pair[r / 2])
-                                    kv.im = -kv.im;
-                                else
-                                    kv = P::kernel(x, nullptr, kps[r]);
-                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y}, kv);
-                            }
-                        }
-                        else
-                        {
-                            const cplx<float> kv = P::kernel(x, nullptr, a.kp);
-#pragma unroll
-                            for (int r = 0; r < NB; r++)
-                                cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y}, kv);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < NB; r++)
-                {
-                    accr[r] += acc[r].re;
-                    acci[r] += acc[r].im;
-                }
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < NB; r++)
-        {
-            rr[r][threadIdx.x] = accr[r];
-            ri[r][threadIdx.x] = acci[r];
-        }
-        __syncthreads();
-        if (active && si == 0)
-        {
-#pragma unroll
-            for (int r = 0; r < NB; r++)
-            {
-                double sr = 0, sim = 0;
-                for (int s = 0; s < S; s++)
-                {
-                    sr += rr[r][ti + s * cnt];
-                    sim += ri[r][ti + s * cnt];
-                }
-                bp.unear[(size_t)(pb + r) * bp.n_tgt + t] = make_double2(sr, sim);
-            }
-        }
-    }
-}
-
 // Enqueues the batched mixed matvec of bp.nrhs (<= bp.groups * BATCH_NB)
 // right-hand sides, one launch per stage and level; returns the number of
 // kernels launched, or -1 when this operator's shape has no batched path
@@ -456,7 +295,8 @@ static int run_mult_batch(const MultPtrs& m, const BatchPtrs& bp, const void* d_
             }
             if (hk)
                 hk->begin(PROF_NEAR);
-            near_batch_kernel<KIND, MK><<<dim3(m.n_tleaf, bp.groups), EVAL_THREADS, 0, ns>>>(ea, bp);
+            near_batch_kernel<KIND, MK, BATCH_NB>
+                <<<dim3(m.n_tleaf, bp.groups), NEAR_THREADS, 0, ns>>>(ea, bp);
             IFGF_CHECK_LAUNCH();
             if (hk)
                 hk->end();

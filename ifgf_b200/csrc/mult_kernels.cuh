@@ -623,18 +623,66 @@ constexpr int EVAL_THREADS = 128;
 // target leaves whose size does not divide the block (leaves of 17-69
 // targets at N = 1e6: 89 % of lanes busy against 77 %).
 constexpr int FAR_THREADS = 256;
-constexpr int EVAL_NEAR = 0, EVAL_FAR = 1; // the two passes of target evaluation
 
-// Near field: one CTA per target leaf.  The leaf's near source boxes hold a
-// few dozen points each, so their ranges are scanned into one sequence and the
-// CTA stages 256 sources of it at a time, the next ones loading while it
+// The sources of a target leaf's near boxes as one sequence (the boxes hold a
+// few dozen points each), for CTAs of NEAR_THREADS threads: near_scan makes the
+// prefix sums pre[0 .. nb] of the sources in nb <= NEAR_THREADS boxes from list
+// position b0 (first: their first sources; every thread calls it),
+// near_source the source at position q of the sequence.
+constexpr int NEAR_THREADS = 256;
+__device__ __forceinline__ void near_scan(const EvalArgs& a, long long b0, int nb, int* pre,
+                                          int* first, int* wsum)
+{
+    const int tid = threadIdx.x;
+    int n = 0, f = 0;
+    if (tid < nb)
+    {
+        const int sb = a.near_src[b0 + tid];
+        f = a.T.box_first[sb];
+        n = a.T.box_last[sb] - f;
+    }
+    int sum = n;
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1)
+    {
+        const int o = __shfl_up_sync(~0u, sum, m);
+        if ((tid & 31) >= m)
+            sum += o;
+    }
+    __syncthreads(); // the previous boxes' tables are no longer read
+    if ((tid & 31) == 31)
+        wsum[tid >> 5] = sum;
+    __syncthreads();
+    for (int w = 0; w < (tid >> 5); w++)
+        sum += wsum[w];
+    pre[tid + 1] = sum;
+    first[tid] = f;
+    if (tid == 0)
+        pre[0] = 0;
+    __syncthreads();
+}
+__device__ __forceinline__ int near_source(const int* pre, const int* first, int nb, int q)
+{
+    int lo = 0, hi = nb; // pre[lo] <= q < pre[hi]
+    while (hi - lo > 1)
+    {
+        const int mid = (lo + hi) >> 1;
+        if (pre[mid] <= q)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return first[lo] + (q - pre[lo]);
+}
+
+// FP64 near field: one CTA per target leaf, 256 near sources staged at a time,
+// the next ones loading while it
 // evaluates; thread (ti, si) takes target ti and every S-th staged source
 // (S = threads / targets), two at a time; the S partial sums are added in a
 // fixed order.  Bound by the FP64 pipe.  Per matvec 6.2 ms at N = 1e6, 1.3 at
 // 2e5, 0.09 at 2e4 (Laplace); staging one box at a time with 128 threads and
 // two barriers a box took 8.5, 2.0 and 0.25 (10.7, 2.6 and 0.40 with the
 // library functions).
-constexpr int NEAR_THREADS = 256;
 template <int KIND>
 __global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_constant__ EvalArgs a)
 {
@@ -660,50 +708,15 @@ __global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_cons
         cplx<double> acc = {0.0, 0.0};
         for (long long b0 = nb0; b0 < nb1; b0 += TH)
         {
-            // prefix sums of the sources in up to TH boxes
             const int nb = (int)min((long long)TH, nb1 - b0);
-            int n = 0, f = 0;
-            if (tid < nb)
-            {
-                const int sb = a.near_src[b0 + tid];
-                f = a.T.box_first[sb];
-                n = a.T.box_last[sb] - f;
-            }
-            int sum = n;
-#pragma unroll
-            for (int m = 1; m < 32; m <<= 1)
-            {
-                const int o = __shfl_up_sync(~0u, sum, m);
-                if ((tid & 31) >= m)
-                    sum += o;
-            }
-            __syncthreads(); // the previous boxes' tables are no longer read
-            if ((tid & 31) == 31)
-                wsum[tid >> 5] = sum;
-            __syncthreads();
-            for (int w = 0; w < (tid >> 5); w++)
-                sum += wsum[w];
-            pre[tid + 1] = sum;
-            first[tid] = f;
-            if (tid == 0)
-                pre[0] = 0;
-            __syncthreads();
+            near_scan(a, b0, nb, pre, first, wsum);
             const int total = pre[nb];
             double2 v0, v1, v2, v3;
             auto fetch = [&](int c) {
                 const int q = c + tid;
                 if (q >= total)
                     return;
-                int lo = 0, hi = nb; // pre[lo] <= q < pre[hi]
-                while (hi - lo > 1)
-                {
-                    const int mid = (lo + hi) >> 1;
-                    if (pre[mid] <= q)
-                        lo = mid;
-                    else
-                        hi = mid;
-                }
-                const int i = first[lo] + (q - pre[lo]);
+                const int i = near_source(pre, first, nb, q);
                 const double2 wv = a.w[i];
                 v0 = make_double2(a.S.sx[i], a.S.sy[i]);
                 v1 = make_double2(a.S.sz[i], wv.x);
@@ -1820,37 +1833,164 @@ static __global__ void __launch_bounds__(256) coarse_to_fine_mixed_kernel(C2FArg
     }
 }
 
-// Mixed-precision target leaf evaluation: near-field terms in FP32 on
-// coordinates relative to the leaf's first target, far-field Chebyshev sums
-// in FP32, every contribution accumulated in FP64.
-template <int KIND, int N0, int N1, int N2, int PART>
-__global__ void __launch_bounds__(PART == EVAL_FAR ? FAR_THREADS : EVAL_THREADS, PART == EVAL_FAR ? 3 : 6)
-    target_eval_mixed_kernel(EvalArgs a)
+// Mixed-precision near field of a plane group (blockIdx.y: NB planes, one for
+// a single right-hand side): one kernel value per (target, source) pair,
+// applied to every plane (with MK one per plane, or per conjugate pair).
+// Sources are staged like in near_kernel, on coordinates relative to the
+// leaf's first target (FP64 ones for the kernels with normals, see
+// PluginF::kernel_d); sums of up to 16 terms in FP32, the rest in FP64.
+// Against staging one box at a time with 128 threads: 0.46 -> 0.29 ms for the
+// single gradient matvec at N = 5e4, 3.6 -> 3.2 at 1e6 (Helmholtz), 9.0 -> 7.2
+// for the 64-wavenumber CQ batch at 1e5.
+template <int KIND, bool MK, int NB>
+__global__ void __launch_bounds__(NEAR_THREADS)
+    near_batch_kernel(const __grid_constant__ EvalArgs a, const __grid_constant__ BatchPtrs bp)
 {
-    constexpr int TH = PART == EVAL_FAR ? FAR_THREADS : EVAL_THREADS;
     using P = PluginF<KIND>;
-    // kernels with normals stage FP64 coordinates (see PluginF::kernel_d)
-    using CT = typename std::conditional<P::needs_normals, double, float>::type;
-    __shared__ CT xs[TH], ys[TH], zs[TH];
-    __shared__ float wr[TH], wi[TH];
-    __shared__ double n0[P::needs_normals ? TH : 1], n1[P::needs_normals ? TH : 1],
-        n2[P::needs_normals ? TH : 1];
-    __shared__ double rr[TH], ri[TH];
-    constexpr int NF = PART == EVAL_FAR ? TH : 1;
-    __shared__ double fcx[NF], fcy[NF], fcz[NF], fH[NF];
-    __shared__ long long ffm[NF];
-    __shared__ int flev[NF];
-    __shared__ LookupF lfs[PART == EVAL_FAR ? MAX_LEVELS : 1];
-    if (PART == EVAL_FAR)
-        for (int l = threadIdx.x; l < a.L; l += blockDim.x)
-            make_lookupf(a.lv[l], lfs[l]); // read after the first chunk's barriers
-    const float2* wf = reinterpret_cast<const float2*>(a.w);
-    const float2* fcf = reinterpret_cast<const float2*>(a.fcoef);
+    constexpr int TH = NEAR_THREADS, FLUSH = 16;
+    constexpr bool NRM = P::needs_normals;
+    using CT = typename std::conditional<NRM, double, float>::type;
+    __shared__ KParams kps[MK ? NB : 1];
+    const int pb = blockIdx.y * NB, tid = threadIdx.x;
+    bool pair[NB / 2 + 1]; // planes 2 h and 2 h + 1 at conjugate wavenumbers
+    if constexpr (MK)
+    {
+        if (tid < NB)
+            kps[tid] = bp.kp_plane[pb + tid]; // read after the chunk barriers
+#pragma unroll
+        for (int h = 0; h < NB / 2; h++)
+            pair[h] = bp.conj_prev && bp.conj_prev[pb + 2 * h + 1];
+    }
+    __shared__ CT xs[3][TH];
+    __shared__ double ns[NRM ? 3 : 1][NRM ? TH : 1];
+    __shared__ float2 ws[NB][TH];
+    __shared__ double2 part[TH];
+    __shared__ int pre[TH + 1], first[TH], wsum[TH / 32];
     const int tl = blockIdx.x;
     const int tf = a.tl_first[tl], tlast = a.tl_last[tl];
     const double r0 = a.tx[tf], r1 = a.ty[tf], r2 = a.tz[tf]; // local origin
-    const long long nb0 = a.near_off[tl], nb1 = PART == EVAL_NEAR ? a.near_off[tl + 1] : nb0;
-    const long long fb0 = a.far_off[tl], fb1 = PART == EVAL_FAR ? a.far_off[tl + 1] : fb0;
+    const long long nb0 = a.near_off[tl], nb1 = a.near_off[tl + 1];
+    for (int base = tf; base < tlast; base += TH)
+    {
+        const int cnt = min(TH, tlast - base);
+        const int S = TH / cnt;
+        const int ti = tid % cnt, si = tid / cnt;
+        const bool active = si < S;
+        const int t = base + ti;
+        const CT y0 = (CT)(a.tx[t] - r0), y1 = (CT)(a.ty[t] - r1), y2 = (CT)(a.tz[t] - r2);
+        double accr[NB], acci[NB];
+#pragma unroll
+        for (int r = 0; r < NB; r++)
+            accr[r] = acci[r] = 0.0;
+        for (long long b0 = nb0; b0 < nb1; b0 += TH)
+        {
+            const int nb = (int)min((long long)TH, nb1 - b0);
+            near_scan(a, b0, nb, pre, first, wsum);
+            const int total = pre[nb];
+            for (int c = 0; c < total; c += TH)
+            {
+                const int ccnt = min(TH, total - c);
+                __syncthreads(); // the previous chunk is no longer read
+                if (tid < ccnt)
+                {
+                    const int i = near_source(pre, first, nb, c + tid);
+                    xs[0][tid] = (CT)(a.S.sx[i] - r0);
+                    xs[1][tid] = (CT)(a.S.sy[i] - r1);
+                    xs[2][tid] = (CT)(a.S.sz[i] - r2);
+#pragma unroll
+                    for (int r = 0; r < NB; r++)
+                        ws[r][tid] = bp.w[(size_t)(pb + r) * bp.n_src + i];
+                    if constexpr (NRM)
+                    {
+                        ns[0][tid] = a.S.nx[i];
+                        ns[1][tid] = a.S.ny[i];
+                        ns[2][tid] = a.S.nz[i];
+                    }
+                }
+                __syncthreads();
+                if (!active)
+                    continue;
+                for (int i0 = si; i0 < ccnt; i0 += FLUSH * S)
+                {
+                    cplx<float> acc[NB];
+#pragma unroll
+                    for (int r = 0; r < NB; r++)
+                        acc[r] = {0.f, 0.f};
+                    const int i1 = min(ccnt, i0 + FLUSH * S);
+                    for (int i = i0; i < i1; i += S)
+                    {
+                        const CT x[3] = {xs[0][i] - y0, xs[1][i] - y1, xs[2][i] - y2};
+                        auto value = [&](const KParams& kp) {
+                            if constexpr (NRM)
+                            {
+                                const double nv[3] = {ns[0][i], ns[1][i], ns[2][i]};
+                                return P::kernel_d(x, nv, kp);
+                            }
+                            else
+                                return P::kernel(x, nullptr, kp);
+                        };
+                        cplx<float> kv = {0.f, 0.f};
+                        if constexpr (!MK)
+                            kv = value(a.kp);
+#pragma unroll
+                        for (int r = 0; r < NB; r++)
+                        {
+                            if constexpr (MK)
+                            {
+                                if (r % 2 == 1 && pair[r / 2])
+                                    kv.im = -kv.im;
+                                else
+                                    kv = value(kps[r]);
+                            }
+                            cfmaf(acc[r], cplx<float>{ws[r][i].x, ws[r][i].y}, kv);
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < NB; r++)
+                    {
+                        accr[r] += acc[r].re;
+                        acci[r] += acc[r].im;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < NB; r++)
+        {
+            __syncthreads(); // the previous plane's sums are no longer read
+            part[tid] = make_double2(accr[r], acci[r]);
+            __syncthreads();
+            if (si == 0)
+            {
+                double sr = 0, sim = 0;
+                for (int s = 0; s < S; s++)
+                {
+                    sr += part[ti + s * cnt].x;
+                    sim += part[ti + s * cnt].y;
+                }
+                bp.unear[(size_t)(pb + r) * bp.n_tgt + t] = make_double2(sr, sim);
+            }
+        }
+    }
+}
+
+// Mixed-precision far field of a single right-hand side, one CTA per target
+// leaf: Chebyshev sums in FP32, every contribution accumulated in FP64.
+template <int KIND, int N0, int N1, int N2>
+__global__ void __launch_bounds__(FAR_THREADS, 3) target_eval_mixed_kernel(EvalArgs a)
+{
+    constexpr int TH = FAR_THREADS;
+    __shared__ double rr[TH], ri[TH];
+    __shared__ double fcx[TH], fcy[TH], fcz[TH], fH[TH];
+    __shared__ long long ffm[TH];
+    __shared__ int flev[TH];
+    __shared__ LookupF lfs[MAX_LEVELS];
+    for (int l = threadIdx.x; l < a.L; l += blockDim.x)
+        make_lookupf(a.lv[l], lfs[l]); // read after the first chunk's barriers
+    const float2* fcf = reinterpret_cast<const float2*>(a.fcoef);
+    const int tl = blockIdx.x;
+    const int tf = a.tl_first[tl], tlast = a.tl_last[tl];
+    const long long fb0 = a.far_off[tl], fb1 = a.far_off[tl + 1];
     for (int base = tf; base < tlast; base += TH)
     {
         const int cnt = min(TH, tlast - base);
@@ -1859,59 +1999,7 @@ __global__ void __launch_bounds__(PART == EVAL_FAR ? FAR_THREADS : EVAL_THREADS,
         const bool active = si < S;
         const int t = base + ti;
         const double y0 = a.tx[t], y1 = a.ty[t], y2 = a.tz[t];
-        const float yl0 = (float)(y0 - r0), yl1 = (float)(y1 - r1), yl2 = (float)(y2 - r2);
         double accr = 0, acci = 0;
-        for (long long e = nb0; e < nb1; e++)
-        {
-            const int sb = a.near_src[e];
-            const int sf = a.T.box_first[sb], sl = a.T.box_last[sb];
-            for (int cs = sf; cs < sl; cs += TH)
-            {
-                const int ccnt = min(TH, sl - cs);
-                __syncthreads();
-                if (threadIdx.x < ccnt)
-                {
-                    const int i = cs + threadIdx.x;
-                    xs[threadIdx.x] = (CT)(a.S.sx[i] - r0);
-                    ys[threadIdx.x] = (CT)(a.S.sy[i] - r1);
-                    zs[threadIdx.x] = (CT)(a.S.sz[i] - r2);
-                    const float2 wv = wf[i];
-                    wr[threadIdx.x] = wv.x;
-                    wi[threadIdx.x] = wv.y;
-                    if (P::needs_normals)
-                    {
-                        n0[threadIdx.x] = a.S.nx[i];
-                        n1[threadIdx.x] = a.S.ny[i];
-                        n2[threadIdx.x] = a.S.nz[i];
-                    }
-                }
-                __syncthreads();
-                if (active)
-                {
-                    cplx<float> acc = {0.f, 0.f};
-                    if constexpr (P::needs_normals)
-                    {
-                        const double yd0 = y0 - r0, yd1 = y1 - r1, yd2 = y2 - r2;
-                        for (int i = si; i < ccnt; i += S)
-                        {
-                            const double x[3] = {xs[i] - yd0, ys[i] - yd1, zs[i] - yd2};
-                            const double nv[3] = {n0[i], n1[i], n2[i]};
-                            cfmaf(acc, cplx<float>{wr[i], wi[i]}, P::kernel_d(x, nv, a.kp));
-                        }
-                    }
-                    else
-                    {
-                        for (int i = si; i < ccnt; i += S)
-                        {
-                            const float x[3] = {xs[i] - yl0, ys[i] - yl1, zs[i] - yl2};
-                            cfmaf(acc, cplx<float>{wr[i], wi[i]}, P::kernel(x, nullptr, a.kp));
-                        }
-                    }
-                    accr += acc.re;
-                    acci += acc.im;
-                }
-            }
-        }
         // far sources in chunks of TH boxes, whose centre, size,
         // level and fine-map row are staged in shared memory first
         for (long long e0 = fb0; e0 < fb1; e0 += TH)
@@ -1961,21 +2049,16 @@ __global__ void __launch_bounds__(PART == EVAL_FAR ? FAR_THREADS : EVAL_THREADS,
                 sr += rr[ti + s * cnt];
                 sim += ri[ti + s * cnt];
             }
-            if (PART == EVAL_NEAR)
-                a.unear[t] = make_double2(sr, sim);
+            const double2 nr = a.unear[t];
+            sr += nr.x;
+            sim += nr.y;
+            const long long o = a.tgt_perm[t];
+            if (a.real_out)
+                a.out[o] = sr;
             else
             {
-                const double2 nr = a.unear[t];
-                sr += nr.x;
-                sim += nr.y;
-                const long long o = a.tgt_perm[t];
-                if (a.real_out)
-                    a.out[o] = sr;
-                else
-                {
-                    a.out[2 * o] = sr;
-                    a.out[2 * o + 1] = sim;
-                }
+                a.out[2 * o] = sr;
+                a.out[2 * o + 1] = sim;
             }
         }
     }
@@ -2090,7 +2173,12 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         if (hk)
             hk->begin(PROF_NEAR);
         if (MIXED)
-            target_eval_mixed_kernel<KIND, 0, 0, 0, EVAL_NEAR><<<m.n_tleaf, EVAL_THREADS, 0, ns>>>(ea);
+        {
+            BatchPtrs bp{};
+            bp.w = reinterpret_cast<float2*>(m.w);
+            bp.unear = m.unear;
+            near_batch_kernel<KIND, false, 1><<<m.n_tleaf, NEAR_THREADS, 0, ns>>>(ea, bp);
+        }
         else
             near_kernel<KIND><<<m.n_tleaf, NEAR_THREADS, 0, ns>>>(ea);
         IFGF_CHECK_LAUNCH();
@@ -2267,7 +2355,7 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         if (by_cone)
             launch_far_gather(m, d_u, real, st);
         else if (MIXED)
-            target_eval_mixed_kernel<KIND, N0, N1, N2, EVAL_FAR><<<m.n_tleaf, FAR_THREADS, 0, st>>>(ea);
+            target_eval_mixed_kernel<KIND, N0, N1, N2><<<m.n_tleaf, FAR_THREADS, 0, st>>>(ea);
         else
         {
             // without the plan; orders above (4, 7, 7) by the runtime-order sums
