@@ -45,8 +45,10 @@ struct KParams
     static constexpr bool NORMAL = false; // squared distances may be zero or subnormal
     double kr, ki; // k = kr + i ki (real kernels use kr)
     int dx;        // GradHelmholtz derivative direction, -1 = plain single layer
-    // kr and ki split into two floats each (hi + lo), for the mixed pipeline
-    float krh, krl, kih, kil;
+    // kr and ki rounded to floats, and the wavenumbers in turns, kr / (2 pi)
+    // and -ki / (2 pi), as two floats each (hi + lo), for the mixed pipeline
+    float krh, kih;
+    float trh, trl, tih, til;
     // FP64 phases and damping in the units their reductions use, as hi + lo
     // pairs: quarter turns 2 kr / pi and -2 ki / pi, octaves -kr / ln 2
     double qrh, qrl, qih, qil, erh, erl;
@@ -66,15 +68,17 @@ inline KParams make_kparams(double kr, double ki, int dx)
     p.ki = ki;
     p.dx = dx;
     p.krh = (float)kr;
-    p.krl = (float)(kr - (double)p.krh);
     p.kih = (float)ki;
-    p.kil = (float)(ki - (double)p.kih);
     // 2 / pi and 1 / ln 2 as hi + lo pairs
     constexpr double TWO_PI_H = 0.6366197723675814, TWO_PI_L = -3.935735335036497e-17;
     constexpr double LOG2E_H = 1.4426950408889634, LOG2E_L = 2.0355273740931033e-17;
     scaled_pair(kr, TWO_PI_H, TWO_PI_L, &p.qrh, &p.qrl);
     scaled_pair(-ki, TWO_PI_H, TWO_PI_L, &p.qih, &p.qil);
     scaled_pair(-kr, LOG2E_H, LOG2E_L, &p.erh, &p.erl);
+    p.trh = (float)(0.25 * p.qrh);
+    p.trl = (float)(0.25 * p.qrh - (double)p.trh);
+    p.tih = (float)(0.25 * p.qih);
+    p.til = (float)(0.25 * p.qih - (double)p.tih);
     return p;
 }
 
@@ -693,55 +697,53 @@ template <> struct Plugin<K_COMBINEDFIELD_DK>
 // ===========================================================================
 constexpr float INV4PIF = (float)INV4PI;
 
-// (cos(k r), sin(k r)) with k r and its reduction in FP64
-__device__ __forceinline__ cplx<float> phase_sc(double k, double r)
+// (cos, sin) of (qh + ql) r quarter turns, formed and reduced in FP64: the
+// nearest multiple of four is taken off exactly by FMA (adding 1.5 2^54 rounds
+// to it), |f| <= 2
+__device__ __forceinline__ cplx<float> phase_sc(double qh, double ql, double r)
 {
-    const double th = k * r;
-    const double n = rint(th * (1.0 / (2.0 * DPI)));
-    const float red = (float)fma(-n, 2.0 * DPI, th);
+    constexpr double MAGIC4 = 4.0 * ROUND_MAGIC;
+    const double n = fma(qh, r, MAGIC4) - MAGIC4;
+    const double f = fma(ql, r, fma(qh, r, -n));
     float s, c;
-    __sincosf(red, &s, &c);
+    __sincosf((float)f * 1.5707963267948966f, &s, &c);
     return {c, s};
 }
 
-// (cos(k r), sin(k r)) for an FP32 distance r, with k r formed and reduced
-// modulo 2 pi in double-float arithmetic: k = kh + kl (two floats, made on the
-// host), the product k r as an unevaluated float pair (exact through FMA) and
-// 2 pi as a three-float sum (Cody-Waite), so the reduced angle carries the
-// accuracy of an FP64 reduction without leaving the FP32 pipes.
-__device__ __forceinline__ cplx<float> phase_sc_ff(float kh, float kl, float r)
+// (cos, sin) of (th + tl) r turns for an FP32 distance r: the nearest integer
+// is taken off exactly by FMA (adding 1.5 2^23 rounds to it), so the reduced
+// angle carries the accuracy of an FP64 reduction without leaving the FP32
+// pipes
+__device__ __forceinline__ cplx<float> phase_sc_ff(float th, float tl, float r)
 {
-    const float th = kh * r;
-    const float tl = fmaf(kh, r, -th) + kl * r;
-    constexpr float C1 = 6.2831854820251465f;      // float(2 pi)
-    constexpr float C2 = -1.7484555314695172e-07f; // float(2 pi - C1)
-    constexpr float C3 = -6.8604980400235275e-15f; // float(2 pi - C1 - C2)
-    const float n = rintf(th * 0.15915493667125702f);
-    float red = fmaf(-n, C1, th);
-    red = fmaf(-n, C2, red);
-    red = fmaf(-n, C3, red) + tl;
+    constexpr float MAGIC = 12582912.f;
+    const float n = fmaf(th, r, MAGIC) - MAGIC;
+    const float f = fmaf(tl, r, fmaf(th, r, -n));
     float s, c;
-    __sincosf(red, &s, &c);
+    __sincosf(f * 6.2831853071795865f, &s, &c);
     return {c, s};
 }
 
 // e^{-k r} for complex k (FP64 distance): e^{-kr r} (cos(ki r), -sin(ki r))
 __device__ __forceinline__ cplx<float> exp_mk_f(const KParams& p, double r)
 {
-    const cplx<float> e = phase_sc(-p.ki, r);
+    const cplx<float> e = phase_sc(p.qih, p.qil, r);
     const float m = __expf((float)(-p.kr * r));
     return {m * e.re, m * e.im};
 }
-__device__ __forceinline__ cplx<float> exp_ik_f(double k, double r) { return phase_sc(k, r); }
+__device__ __forceinline__ cplx<float> exp_ik_f(const KParams& p, double r)
+{
+    return phase_sc(p.qrh, p.qrl, r);
+}
 
 // the same for an FP32 distance (double-float phase)
 __device__ __forceinline__ cplx<float> exp_ik_ff(const KParams& p, float r)
 {
-    return phase_sc_ff(p.krh, p.krl, r);
+    return phase_sc_ff(p.trh, p.trl, r);
 }
 __device__ __forceinline__ cplx<float> exp_mk_ff(const KParams& p, float r)
 {
-    const cplx<float> e = phase_sc_ff(-p.kih, -p.kil, r);
+    const cplx<float> e = phase_sc_ff(p.tih, p.til, r);
     const float m = __expf(-p.krh * r);
     return {m * e.re, m * e.im};
 }
@@ -999,10 +1001,10 @@ template <> struct PluginF<K_COMBINEDFIELD_DK>
 template <int KIND>
 __device__ __forceinline__ cplx<float> cf_mixed(double d2, const KParams& p)
 {
-    const double d = sqrt(d2);
+    const double d = dist_inv<false>(d2).d;
     if (KIND == K_HELMHOLTZ_DK || KIND == K_COMBINEDFIELD_DK)
     {
-        const cplx<float> e = exp_ik_f(p.kr, d);
+        const cplx<float> e = exp_ik_f(p, d);
         return {e.re * INV4PIF, e.im * INV4PIF};
     }
     const float id = rsqrtf((float)d2) * INV4PIF;
@@ -1010,7 +1012,7 @@ __device__ __forceinline__ cplx<float> cf_mixed(double d2, const KParams& p)
         return {id, 0.f};
     if (KIND == K_HELMHOLTZ || KIND == K_COMBINEDFIELD)
     {
-        const cplx<float> e = exp_ik_f(p.kr, d);
+        const cplx<float> e = exp_ik_f(p, d);
         return {e.re * id, e.im * id};
     }
     const cplx<float> e = exp_mk_f(p, d);
@@ -1022,13 +1024,13 @@ __device__ __forceinline__ cplx<float> transfer_mixed(double d2, double dp2, con
 {
     const double d = sqrt(d2), dp = sqrt(dp2);
     if (KIND == K_HELMHOLTZ_DK || KIND == K_COMBINEDFIELD_DK)
-        return exp_ik_f(p.kr, d - dp);
+        return exp_ik_f(p, d - dp);
     const float ratio = __fdividef((float)dp, (float)d);
     if (KIND == K_LAPLACE)
         return {ratio, 0.f};
     if (KIND == K_HELMHOLTZ || KIND == K_COMBINEDFIELD)
     {
-        const cplx<float> e = exp_ik_f(p.kr, d - dp);
+        const cplx<float> e = exp_ik_f(p, d - dp);
         return {e.re * ratio, e.im * ratio};
     }
     const cplx<float> e = exp_mk_f(p, d - dp);
