@@ -1083,40 +1083,43 @@ __device__ __forceinline__ void make_lookupf(const LevelGeom& G, LookupF& L)
     }
 }
 
-// fine_lookup_mixed with the level's FP32 parameters at hand: with
-// t = (s - lo) / h the element index is q = floor(t) (clamped) and the local
-// coordinate 2 (t - q) - 1, the same quantities as (s - centre) / (h / 2).
-// The FP64 fallback (outside the FP32 domain or an inactive cone) is that of
-// fine_lookup_mixed.
-__device__ __forceinline__ int fine_lookup_fast(const LookupF& L, const LevelGeom& G,
-                                                const int* __restrict__ fm, const double* p,
-                                                double H, float* loc, unsigned long long* err)
+// Fine element of the point p in FP32 (-1 outside the domain) and its local
+// coordinates: with t = (s - lo) / h the element index is q = floor(t)
+// (clamped) and the local coordinate 2 (t - q) - 1, the same quantities as
+// (s - centre) / (h / 2).  Roundings are spelled out, so that every kernel that
+// looks a pair up gets the same coordinates.
+__device__ __forceinline__ int lookup_f(const LookupF& L, const double* p, double H, float* loc)
 {
     float sf[3];
     cart_to_interp_f((float)p[0], (float)p[1], (float)p[2], (float)H, sf);
     bool inside = true;
     int id = 0, stride = 1;
-    float fr[3];
 #pragma unroll
     for (int j = 0; j < 3; j++)
     {
         inside = inside && sf[j] >= L.lo[j] && sf[j] <= L.hi[j];
-        const float t = (sf[j] - L.lo[j]) * L.hinv[j];
+        const float t = __fmul_rn(__fsub_rn(sf[j], L.lo[j]), L.hinv[j]);
         const float q = fminf(fmaxf(floorf(t), 0.f), L.top[j]);
-        fr[j] = t - q;
+        loc[j] = __fmaf_rn(2.f, __fsub_rn(t, q), -1.f);
         id += __float2int_rz(q) * stride;
         stride *= L.nf[j];
     }
-    if (inside)
+    return inside ? id : -1;
+}
+
+// fine_lookup_mixed with the level's FP32 parameters at hand (lookup_f); the
+// FP64 fallback (outside the FP32 domain or an inactive cone) is that of
+// fine_lookup_mixed.
+__device__ __forceinline__ int fine_lookup_fast(const LookupF& L, const LevelGeom& G,
+                                                const int* __restrict__ fm, const double* p,
+                                                double H, float* loc, unsigned long long* err)
+{
+    const int id = lookup_f(L, p, H, loc);
+    if (id >= 0)
     {
         const int gf = fm[id];
         if (gf >= 0)
-        {
-#pragma unroll
-            for (int d = 0; d < 3; d++)
-                loc[d] = fmaf(2.f, fr[d], -1.f);
             return gf;
-        }
     }
     double s[3], ld[3];
     cart_to_interp(p[0], p[1], p[2], H, s);

@@ -24,16 +24,25 @@ constexpr int THREADS = 256;
 
 // One CTA per target leaf, one thread per (far box, target) pair: the pair's
 // fine cone (the FP64 lookup that marked the active cones,
-// ifgfoperator.hpp:1736-1891), its index in pos, and the pairs of every cone
-// counted, lanes of one cone together.
+// ifgfoperator.hpp:1736-1891; mixed: the FP32 lookup of the mixed far
+// kernels), its index in pos, and the pairs of every cone counted, lanes of
+// one cone together.
+template <bool MIXED>
 __global__ void __launch_bounds__(THREADS)
     count_kernel(const LevelGeom* __restrict__ lv, TreeArgs T, const double* __restrict__ tx,
                  const double* __restrict__ ty, const double* __restrict__ tz,
                  const int* __restrict__ fmap, const int* __restrict__ tl_first,
                  const int* __restrict__ tl_last, const long long* __restrict__ far_off,
                  const int* __restrict__ far_src, const long long* __restrict__ leaf_off, int* pos,
-                 int* count, unsigned long long* err)
+                 int* count, unsigned long long* err, int L)
 {
+    __shared__ LookupF lfs[MIXED ? MAX_LEVELS : 1];
+    if (MIXED)
+    {
+        for (int l = threadIdx.x; l < L; l += blockDim.x)
+            make_lookupf(lv[l], lfs[l]);
+        __syncthreads();
+    }
     const int tl = blockIdx.x;
     const int t0 = tl_first[tl], cnt = tl_last[tl] - t0;
     const long long f0 = far_off[tl], n = (far_off[tl + 1] - f0) * cnt, o = leaf_off[tl];
@@ -44,17 +53,28 @@ __global__ void __launch_bounds__(THREADS)
         if (q < n)
         {
             const int sb = far_src[f0 + q / cnt], t = t0 + (int)(q % cnt);
-            const LevelGeom& G = lv[T.box_level[sb]];
-            double s[3];
-            cart_to_interp(tx[t] - T.box_c[3 * sb], ty[t] - T.box_c[3 * sb + 1],
-                           tz[t] - T.box_c[3 * sb + 2], T.box_H[sb], s);
-            const int fe = element_for_point(s, G.dmin, G.dmax, G.hfi, G.nf);
-            if (fe >= 0)
+            const int lev = T.box_level[sb];
+            const LevelGeom& G = lv[lev];
+            const double p[3] = {tx[t] - T.box_c[3 * sb], ty[t] - T.box_c[3 * sb + 1],
+                                 tz[t] - T.box_c[3 * sb + 2]};
+            const long long nft = (long long)G.nf[0] * G.nf[1] * G.nf[2];
+            const int* fm = fmap + G.fmap_off + (long long)(sb - G.box_off) * nft;
+            if (MIXED)
             {
-                const long long nft = (long long)G.nf[0] * G.nf[1] * G.nf[2];
-                gf = fmap[G.fmap_off + (long long)(sb - G.box_off) * nft + fe];
-                if (gf < 0)
-                    atomicAdd(err, 1ull);
+                float loc[3];
+                gf = fine_lookup_fast(lfs[lev], G, fm, p, T.box_H[sb], loc, err);
+            }
+            else
+            {
+                double s[3];
+                cart_to_interp(p[0], p[1], p[2], T.box_H[sb], s);
+                const int fe = element_for_point(s, G.dmin, G.dmax, G.hfi, G.nf);
+                if (fe >= 0)
+                {
+                    gf = fm[fe];
+                    if (gf < 0)
+                        atomicAdd(err, 1ull);
+                }
             }
             pos[o + q] = gf;
         }
@@ -107,6 +127,12 @@ __global__ void tile_kernel(const int* __restrict__ off, int n, int* tile_cone)
             tile_cone[k] = i;
 }
 
+__global__ void lookup_kernel(const LevelGeom* __restrict__ lv, int L, LookupF* out)
+{
+    for (int l = threadIdx.x; l < L; l += blockDim.x)
+        make_lookupf(lv[l], out[l]);
+}
+
 __global__ void meta_kernel(const int* __restrict__ box, const int* __restrict__ el, int n,
                             int2* meta)
 {
@@ -130,7 +156,7 @@ struct Layout
 {
     long long n_fine = 0, pairs = 0, most = 0;
     size_t bytes = 0, scan_b = 0, count_b = 0;
-    size_t val, pos, tgt, tile, meta, host, leaf, trig, lev;
+    size_t val, pos, tgt, tile, meta, lookup, host, leaf, trig, lev;
     bool fits = false; // there are pairs, and fewer than 2^31 places
     explicit Layout(const FarConeBuild& b)
     {
@@ -154,11 +180,13 @@ struct Layout
             return at;
         };
         count_b = ((size_t)(n_fine + 1) * sizeof(int) + 255) / 256 * 256;
-        val = place(std::max((size_t)most * sizeof(double2), 2 * count_b + scan_b));
+        const size_t value_b = b.mixed ? sizeof(float2) : sizeof(double2);
+        val = place(std::max((size_t)most * value_b, 2 * count_b + scan_b));
         pos = place((size_t)pairs * sizeof(int));
         tgt = place((size_t)most * sizeof(int));
         tile = place((size_t)most / FAR_TILE * sizeof(int));
         meta = place((size_t)n_fine * sizeof(int2));
+        lookup = place(b.lv->size() * sizeof(LookupF));
         host = bytes; // from here on filled on the host
         leaf = place(b.leaf_off->size() * sizeof(long long));
         trig = place(n_trig * sizeof(double2));
@@ -244,13 +272,15 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
     size_t scan_b = at.scan_b;
     IFGF_CUDA(cudaMemsetAsync(count, 0, (n_fine + 1) * sizeof(int), nullptr));
     IFGF_CUDA(cudaMemsetAsync(tgt, 0xff, at.meta - at.tgt, nullptr)); // and the tiles
+    lookup_kernel<<<1, 32>>>(b.lv_dev, L, (LookupF*)(m + at.lookup));
     for (int l = 0; l < L; l++)
         if (lv[l].n_fine > 0)
             meta_kernel<<<blocks_for(lv[l].n_fine), 256>>>(b.cone_box[l], b.cone_el[l],
                                                            (int)lv[l].n_fine,
                                                            meta + lv[l].fine_off);
-    count_kernel<<<nl, THREADS>>>(b.lv_dev, b.T, b.tx, b.ty, b.tz, b.fmap, b.tl_first, b.tl_last,
-                                  b.far_off, b.far_src, leaf_off, pos, count, b.err);
+    const auto count_pairs = b.mixed ? count_kernel<true> : count_kernel<false>;
+    count_pairs<<<nl, THREADS>>>(b.lv_dev, b.T, b.tx, b.ty, b.tz, b.fmap, b.tl_first, b.tl_last,
+                                 b.far_off, b.far_src, leaf_off, pos, count, b.err, L);
     pad_kernel<<<blocks_for(n_fine), 256>>>(count, (int)n_fine);
     IFGF_CUDA(cub::DeviceScan::ExclusiveSum(m + at.val + 2 * at.count_b, scan_b, count, off,
                                             (int)n_fine + 1));
@@ -277,7 +307,8 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
                          (const double2*)(m + at.trig),
                          pos,
                          leaf_off,
-                         (double2*)(m + at.val)};
+                         m + at.val,
+                         (const LookupF*)(m + at.lookup)};
     plan.ready = true;
     plan.ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - start)
                   .count();
@@ -286,7 +317,8 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
 // One CTA per target leaf: thread (ti, si) adds the values of target ti over
 // far boxes si, si + S, ... (S = threads / targets); the S sums and the near
 // sum are added in a fixed order and written in the caller's order.  Bound
-// by memory (20 bytes a pair).
+// by memory (20 bytes a pair, mixed 12).
+template <typename V>
 __global__ void __launch_bounds__(THREADS)
     far_gather_kernel(FarConePtrs fc, const int* __restrict__ tl_first,
                       const int* __restrict__ tl_last, const long long* __restrict__ far_off,
@@ -306,15 +338,23 @@ __global__ void __launch_bounds__(THREADS)
         if (si < S)
         {
             const int* pos = fc.pos + fc.leaf_off[tl] + base + ti;
-#pragma unroll 4
-            for (int e = si; e < nbox; e += S)
+            // eight places, then their values, in flight together
+            constexpr int U = 8;
+            for (int e = si; e < nbox; e += U * S)
             {
-                const int at = pos[(long long)e * all];
-                if (at >= 0)
+                int at[U];
+                V v[U];
+#pragma unroll
+                for (int k = 0; k < U; k++)
+                    at[k] = e + k * S < nbox ? pos[(long long)(e + k * S) * all] : -1;
+#pragma unroll
+                for (int k = 0; k < U; k++)
+                    v[k] = at[k] >= 0 ? static_cast<const V*>(fc.val)[at[k]] : V{0, 0};
+#pragma unroll
+                for (int k = 0; k < U; k++)
                 {
-                    const double2 v = fc.val[at];
-                    acc.x += v.x;
-                    acc.y += v.y;
+                    acc.x += (double)v[k].x;
+                    acc.y += (double)v[k].y;
                 }
             }
         }
@@ -342,9 +382,9 @@ __global__ void __launch_bounds__(THREADS)
 
 void launch_far_gather(const MultPtrs& m, void* d_u, bool real, cudaStream_t st)
 {
-    far_gather_kernel<<<m.n_tleaf, THREADS, 0, st>>>(m.fc, m.tl_first, m.tl_last, m.tl_far_off,
-                                                     m.unear, m.tgt_perm, (double*)d_u,
-                                                     real ? 1 : 0);
+    const auto kern = m.mixed ? far_gather_kernel<float2> : far_gather_kernel<double2>;
+    kern<<<m.n_tleaf, THREADS, 0, st>>>(m.fc, m.tl_first, m.tl_last, m.tl_far_off, m.unear,
+                                        m.tgt_perm, (double*)d_u, real ? 1 : 0);
 }
 
 } // namespace ifgf

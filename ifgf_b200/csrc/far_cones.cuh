@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(FAR_CONE_THREADS)
         return;
     const int cone = a.fc.tile_cone[4 * group + (lane >> 3)]; // -1 past the last tile
     const long long place = 32 * group + lane;
-    const int t = cone >= 0 ? a.fc.tgt[place] : -1; // -1: padding
+    const int t = a.fc.tgt[place]; // -1: padding
     // the tiles' coefficient blocks on their way to L1
     for (int q = 0; q < 4; q++)
     {
@@ -275,7 +275,73 @@ __global__ void __launch_bounds__(FAR_CONE_THREADS)
     {
         const cplx<double> f = Plugin<KIND>::cf(D, a.kp);
         const double2 v = vs[warp][lane];
-        a.fc.val[place] = REAL ? make_double2(v.x * f.re, 0.0)
-                               : make_double2(v.x * f.re - v.y * f.im, v.x * f.im + v.y * f.re);
+        static_cast<double2*>(a.fc.val)[place] =
+            REAL ? make_double2(v.x * f.re, 0.0)
+                 : make_double2(v.x * f.re - v.y * f.im, v.x * f.im + v.y * f.re);
     }
+}
+
+// The same for the mixed pipeline, one thread per two places of a tile: the
+// FP32 lookup's local coordinates, FP32 coefficients and sums; every coefficient
+// load serves both places, and the lanes of a tile read one block.  At N = 1e6,
+// p = 9 11.1 ms per matvec with the gather; looking every pair up and
+// reading each lane's block took 17.0, one place per thread 14.5 (L1 73 % busy).
+constexpr int FAR_CONE_PER = 2;
+template <int KIND, int N0, int N1, int N2>
+__global__ void __launch_bounds__(FAR_CONE_THREADS)
+    far_cone_mixed_kernel(const __grid_constant__ FarConeArgs a)
+{
+    constexpr int P_LO = N0 * N1 * N2, R = FAR_CONE_PER;
+    const long long place = (blockIdx.x * (long long)FAR_CONE_THREADS + threadIdx.x) * R;
+    if (place >= 32 * a.fc.n_groups)
+        return;
+    const int cone = a.fc.tile_cone[place / FAR_TILE]; // -1 past the last tile
+    int t[R];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        t[r] = a.fc.tgt[place + r]; // -1: padding
+    const float2* blk = reinterpret_cast<const float2*>(a.fcoef) + (size_t)max(cone, 0) * P_LO;
+    if (cone >= 0) // the block's lines on their way to L1
+        for (int o = 128 * (threadIdx.x % (FAR_TILE / R)); o < P_LO * (int)sizeof(float2);
+             o += 128 * (FAR_TILE / R))
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(blk) + o));
+    bool any = false;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        any |= t[r] >= 0;
+    if (!any)
+        return;
+    const int2 be = a.fc.meta[cone];
+    const int box = be.x, lev = a.T.box_level[box];
+    const double H = a.T.box_H[box];
+    const double xc[3] = {a.T.box_c[3 * box], a.T.box_c[3 * box + 1], a.T.box_c[3 * box + 2]};
+    float loc[R][3], vr[R], vi[R];
+    double d2[R];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+    {
+        const int tr = t[r] >= 0 ? t[r] : 0;
+        const double p[3] = {a.tx[tr] - xc[0], a.ty[tr] - xc[1], a.tz[tr] - xc[2]};
+        d2[r] = p[0] * p[0] + p[1] * p[1] + p[2] * p[2];
+        if (lookup_f(a.fc.lookup[lev], p, H, loc[r]) != be.y && t[r] >= 0)
+        {
+            // a pair that the FP64 lookup placed
+            const LevelGeom& G = a.lv[lev];
+            double s[3], ld[3];
+            cart_to_interp(p[0], p[1], p[2], H, s);
+            to_local(be.y, s, G.dmin, G.hf, G.hfi, G.nf, ld);
+            loc[r][0] = (float)ld[0];
+            loc[r][1] = (float)ld[1];
+            loc[r][2] = (float)ld[2];
+        }
+    }
+    ChebMulti<float, N0, N1, N2, R>::eval(blk, loc, nullptr, vr, vi);
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (t[r] >= 0)
+        {
+            const cplx<float> f = cf_mixed<KIND>(d2[r], a.kp);
+            reinterpret_cast<float2*>(a.fc.val)[place + r] =
+                make_float2(vr[r] * f.re - vi[r] * f.im, vr[r] * f.im + vi[r] * f.re);
+        }
 }

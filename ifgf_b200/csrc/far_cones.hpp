@@ -1,5 +1,5 @@
 // Far-cone plan: the (target, far box) pairs of an operator sorted by the fine
-// cone they evaluate, for the FP64 far field (far_cones.cuh).
+// cone they evaluate, for the far field of the single matvec (far_cones.cuh).
 #pragma once
 
 #include <vector>
@@ -39,6 +39,7 @@ struct FarConeBuild
     // fine cones of every level: box, element (device arrays)
     std::vector<const int*> cone_box, cone_el;
     unsigned long long* err;
+    bool mixed = false; // lookups of the mixed pipeline
 };
 
 // A plan is one allocation.  Small ones (up to FAR_CONES_RESERVE) get it with

@@ -131,7 +131,8 @@ struct FarConePtrs
     const double2* trig = nullptr;  // per level (sin, cos) of the theta, then the phi centres
     const int* pos = nullptr;       // per target leaf [far box][target]: place, or -1
     const long long* leaf_off = nullptr; // first pos entry of every target leaf
-    double2* val = nullptr;         // value of every place
+    void* val = nullptr;            // value of every place: double2, mixed float2
+    const LookupF* lookup = nullptr; // per level: FP32 lookup parameters
 };
 
 // Everything one matvec launch needs (device pointers, sizes, orders).
@@ -178,7 +179,7 @@ struct MultPtrs
     // the upward-kernel autotuner's per-level choice for single-plane
     // matvecs (host array of L: 1 tensor cores, 0 FFMA, -1 none yet)
     const signed char* up_choice = nullptr;
-    // far-cone plan of the FP64 far field (null: the
+    // far-cone plan of the far field (null: the
     // far kernel looks up every pair's cone)
     FarConePtrs fc;
 };
@@ -375,7 +376,8 @@ int launch_mult_batch_kernels(const MultPtrs& m, const BatchPtrs& bp, const void
 // the FFMA and the tensor-core upward transfer of one launch over `planes`
 // right-hand-side planes (bp null: the single-plane buffers of m) are timed
 // on the operator's own tables and buffers (each kernel once to warm up,
-// then the better of two timed launches); choice[l] = 1 where the tensor
+// then once, or the better of two launches of less than 0.5 ms);
+// choice[l] = 1 where the tensor
 // cores were faster by more than 3 %, 0 elsewhere, -1 on levels without
 // both kernels; ms_ffma / ms_tc receive the times (0 where not timed).
 // The buffers' contents are left unspecified (the next matvec rewrites

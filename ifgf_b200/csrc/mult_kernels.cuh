@@ -2338,13 +2338,15 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         if (hk)
             hk->begin(PROF_EVAL);
         bool by_cone = false;
-        if constexpr (!MIXED && N0 > 0)
+        if constexpr (N0 > 0)
             if (m.fc.tile_cone)
             {
                 const FarConeArgs fa{m.fc, m.lv_dev, m.T, m.tx, m.ty, m.tz, m.fcoef, m.kp};
-                constexpr int WARPS = FAR_CONE_THREADS / 32;
-                far_cone_kernel<KIND, N0, N1, N2>
-                    <<<(unsigned)((m.fc.n_groups - 1) / WARPS + 1), FAR_CONE_THREADS, 0, st>>>(fa);
+                // groups of 32 places per CTA
+                constexpr int PER = FAR_CONE_THREADS / 32 * (MIXED ? FAR_CONE_PER : 1);
+                const auto kern = MIXED ? far_cone_mixed_kernel<KIND, N0, N1, N2>
+                                        : far_cone_kernel<KIND, N0, N1, N2>;
+                kern<<<(unsigned)((m.fc.n_groups - 1) / PER + 1), FAR_CONE_THREADS, 0, st>>>(fa);
                 IFGF_CHECK_LAUNCH();
                 launches++;
                 by_cone = true;

@@ -74,7 +74,7 @@ struct DeviceState
     double fp_ovf_few = 0; // share of the records beyond the smaller slot count tried
     bool fp_ready = false;
     double fp_ms = 0;
-    FarConePlan fc; // far-cone plan of the FP64 matvec
+    FarConePlan fc[2]; // far-cone plans of the single matvec (FP64, mixed)
     std::vector<long long> tl_pair_off; // first (far box, target) pair of every target leaf
     DevBuf<double2> w, cvals, fcoef, unear;
     // planes of the batched mixed matvec, allocated on first use for
@@ -1285,7 +1285,8 @@ void Operator::setup_device(const double* normals)
     D.fp_slot.release();
     D.fp_nchunk = 0;
     D.fp_ready = false;
-    D.fc.release();
+    for (FarConePlan& fc : D.fc)
+        fc.release();
     phase("target_leaf_lists");
     // ---- active cones (octree.hpp:351-816) on the GPU ----
     int64_t fmap_total = 0;
@@ -1616,7 +1617,7 @@ void Operator::setup_device(const double* normals)
     if (D.c2f_smem > 220 * 1024)
         throw Error(ERR_INVALID, "interpolation order too high for the coarse-to-fine kernel");
     if (precision_ == PREC_FP64 && far_plan_on_ && far_cone_shape(lo_))
-        reserve_far_cones(far_cone_build(D, lv_), D.fc);
+        reserve_far_cones(far_cone_build(D, lv_), D.fc[0]);
     phase("buffers");
 }
 
@@ -1819,10 +1820,11 @@ void Operator::set_far_plan(bool on)
         D.fp_slot.release();
         D.fp_nchunk = 0;
         D.fp_ready = false;
-        // a captured graph may still read the far-cone plan: kept until the
+        // a captured graph may still read a far-cone plan: kept until the
         // next init
-        if (!D.fc.captured)
-            D.fc.release();
+        for (FarConePlan& fc : D.fc)
+            if (!fc.captured)
+                fc.release();
     }
 }
 
@@ -1838,16 +1840,18 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
         cap = cudaStreamCaptureStatusActive;
     }
     const bool capturing = cap != cudaStreamCaptureStatusNone;
-    if (!D.fc.ready && !D.fc.refused && !capturing)
+    FarConePlan& fc = D.fc[precision_ == PREC_MIXED];
+    if (!fc.ready && !fc.refused && !capturing)
     {
         IFGF_CUDA(cudaSetDevice(device_));
-        const FarConeBuild b = far_cone_build(D, lv_);
-        build_far_cones(b, D.fc);
+        FarConeBuild b = far_cone_build(D, lv_);
+        b.mixed = precision_ == PREC_MIXED;
+        build_far_cones(b, fc);
     }
-    if (!D.fc.ready)
+    if (!fc.ready)
         return;
-    D.fc.captured |= capturing;
-    m.fc = D.fc.p;
+    fc.captured |= capturing;
+    m.fc = fc.p;
 }
 
 void Operator::ensure_far_plan()
@@ -2363,8 +2367,7 @@ void Operator::launch_mult(const void* d_w, void* d_u, void* stream, bool timed,
     }
     MultPtrs m;
     fill_mult_ptrs(m, vkind >= 0);
-    if (precision_ == PREC_FP64)
-        ensure_far_cones(m, stream);
+    ensure_far_cones(m, stream);
     EventHooks log(D, st);
     const bool on = profiling_ || timed;
     int launches = 0;
@@ -3046,9 +3049,10 @@ std::string Operator::stats_json() const
       << (dev_->fp_group.n * sizeof(FarGroup) + dev_->fp_rec.n * sizeof(FarPlanRec) +
           dev_->fp_slot.n * sizeof(int) + dev_->fp_chunk.n * sizeof(FarChunk))
       << ",\"slots_per_group\":" << dev_->fp_nslot << ",\"overflow_share_at_few_slots\":" << dev_->fp_ovf_few << ",\"build_ms\":" << dev_->fp_ms << "}";
-    o << ",\"far_cones\":{\"built\":" << (dev_->fc.ready ? 1 : 0)
-      << ",\"pairs\":" << dev_->fc.pairs << ",\"places\":" << dev_->fc.places
-      << ",\"bytes\":" << dev_->fc.mem.n << ",\"build_ms\":" << dev_->fc.ms << "}";
+    const FarConePlan& fc = dev_->fc[precision_ == PREC_MIXED];
+    o << ",\"far_cones\":{\"built\":" << (fc.ready ? 1 : 0) << ",\"pairs\":" << fc.pairs
+      << ",\"places\":" << fc.places << ",\"bytes\":" << fc.mem.n << ",\"build_ms\":" << fc.ms
+      << "}";
     o << ",\"upward_images_bytes\":[";
     for (int l = 0; l < (int)lv_.size(); l++)
         o << (l ? "," : "") << (l < (int)dev_->tc_img.size() ? dev_->tc_img[l].n : 0);

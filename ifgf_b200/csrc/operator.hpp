@@ -137,8 +137,8 @@ class Operator
     // finds its cones itself (no plan memory)
     void ensure_far_plan();
     void set_batch_far(BatchPtrs& bp);
-    // far-cone plan of the FP64 matvec (built on first use, once per init; not
-    // while `stream` is being captured)
+    // far-cone plan of the single matvec in this precision (built on first
+    // use, once per init; not while `stream` is being captured)
     void ensure_far_cones(MultPtrs& m, void* stream);
     void ensure_upward_tuned(int planes, const BatchPtrs* bp, void* stream);
     // basis images of the tensor-core upward transfer (built on first use of

@@ -108,13 +108,14 @@ int ifgf_set_upward_path(ifgf_operator* op, int path);
  * so that every later matvec skips the lookups (evaluateFromInterp,
  * ifgfoperator.hpp:1736-1891, done as a lookup pass at setup and a sum pass
  * per matvec).  enable = 0 frees the plan and the far kernel looks the cones
- * up in every matvec (same results).  The FP64 matvec keeps a plan of its own
- * (pairs sorted by cone, a value array; about 25 bytes per pair: 9.8 GB at
- * that size, "far_cones" in the stats), built on its first call outside a
+ * up in every matvec (same results).  The single-right-hand-side matvecs
+ * keep plans of their own, one per precision used (pairs sorted by cone, a
+ * value array; about 25 bytes per pair in FP64, 17 mixed: 9.8 and 6.7 GB at
+ * that size, "far_cones" in the stats), built on the first call outside a
  * stream capture where it takes at most a quarter of the free device memory;
- * without it the far kernel looks the cones up (same results to FP64
- * rounding).  enable = 0 frees that too, unless a capture has recorded it (then
- * the next init does).  No reference counterpart. */
+ * without it the far kernel looks the cones up (same results to rounding).
+ * enable = 0 frees them too, unless a capture has recorded one (then the next
+ * init does).  No reference counterpart. */
 int ifgf_set_far_plan(ifgf_operator* op, int enable);
 
 /* Diagnostic of the bounded waits the tensor-core kernels use: launches a

@@ -1,8 +1,9 @@
-"""The far-cone plan of the FP64 matvec (pairs sorted by fine cone, sums on the
-FP64 tensor cores) against the far kernel that looks every pair up.  Both
-evaluate the same interpolants; the local coordinates are formed from other
-roundings (a few 1e-16, amplified by the degree squared and the cone count),
-so the results agree to 1e-12 of their norm, the parity tolerance.
+"""The far-cone plans of the single matvec (pairs sorted by fine cone) against
+the far kernels that look every pair up.  Both evaluate the same interpolants.
+FP64 (sums on the FP64 tensor cores): the local coordinates are formed from
+other roundings (a few 1e-16, amplified by the degree squared and the cone
+count), so the results agree to 1e-12 of their norm, the parity tolerance.
+Mixed: the same FP32 coordinates and terms, summed in another order.
 """
 import numpy as np
 import pytest
@@ -12,6 +13,7 @@ from ifgf_b200 import workloads as W
 from .helpers import KERNELS, densities_for, init_op, make_gpu_op, rel2
 
 TOL = 1e-12
+TOL_MIXED = 1e-6
 
 
 def _both(op, w):
@@ -111,3 +113,33 @@ def test_capture():
         torch.cuda.synchronize()
         assert float((u - ref).norm() / ref.norm()) <= TOL
     del first, second
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", list(KERNELS))
+@pytest.mark.parametrize("order", [8, 9, 10, 12])
+def test_mixed(name, order):
+    n = 4001
+    pts = W.sphere_points(n, seed=0)
+    g = make_gpu_op(name, leaf=40, order=order)
+    init_op(g, name, pts, pts)
+    g.set_precision("mixed")
+    g.set_upward_path("ffma")  # the autotuner's choice would be timed again
+    u, ref, st = _both(g, densities_for(name, n))
+    assert st["built"] == 1
+    assert rel2(u, ref) <= TOL_MIXED, rel2(u, ref)
+
+
+@pytest.mark.gpu
+def test_both_precisions_keep_their_plans():
+    n = 3000
+    pts = W.sphere_points(n, seed=0)
+    w = W.densities(n, seed=1)
+    g = make_gpu_op("helmholtz", leaf=50, order=8)
+    g.init(pts, pts)
+    u = g.mult(w)
+    g.set_precision("mixed")
+    um = g.mult(w)
+    assert rel2(um, u) <= 2e-5
+    g.set_precision("fp64")
+    assert np.array_equal(g.mult(w), u)
