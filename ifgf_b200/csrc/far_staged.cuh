@@ -1,8 +1,8 @@
 // Far-field evaluation with coefficient blocks staged in shared memory, for
 // the batched mixed pipeline (NP = BATCH_NB planes per CTA).  A single plane
 // does not pay for the staging (the per-box work is a quarter, the hashing,
-// copies and barriers are not): the single right-hand-side pipeline keeps its
-// direct kernel.  Included by mult_kernels.cuh inside namespace ifgf, after
+// copies and barriers are not): the single right-hand-side pipeline goes cone
+// by cone (far_cones.cuh).  Included by mult_kernels.cuh inside namespace ifgf, after
 // the evaluation helpers.
 #pragma once
 

@@ -12,9 +12,12 @@
 //     coarse_to_fine    chebtransform, coarseToFine and the fine chebtransform
 //                       (ifgfoperator.hpp:1087-1124, 1539-1637) as three
 //                       per-dimension matrix products
-//   target_eval         per target leaf: near field + far field of every
-//                       admissible source box, written in caller order
-//                       (ifgfoperator.hpp:900-1012, 1707-1891, 862-866)
+//   near                per target leaf: sums over the near source boxes
+//                       (ifgfoperator.hpp:900-1012), beside the level loop
+//   far                 far field of every admissible source box, cone by cone
+//                       with the far-cone plan (far_cones.cuh), else per target
+//                       leaf (target_eval); near sums added, written in caller
+//                       order (ifgfoperator.hpp:1707-1891, 862-866)
 //
 // Included by one translation unit per kernel plug-in (kernels_k<KIND>.cu).
 #pragma once

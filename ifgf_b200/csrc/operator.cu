@@ -1833,19 +1833,30 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
     DeviceState& D = *dev_;
     if (!far_plan_on_ || D.n_tleaf == 0 || !far_cone_shape(lo_))
         return;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess)
-    {
+    // the build allocates and runs on the legacy stream: not while `stream` is
+    // captured, nor while any stream is that the legacy one synchronises with
+    auto captures = [](cudaStream_t st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) == cudaSuccess)
+            return cap != cudaStreamCaptureStatusNone;
         cudaGetLastError();
-        cap = cudaStreamCaptureStatusActive;
-    }
-    const bool capturing = cap != cudaStreamCaptureStatusNone;
+        return true;
+    };
+    const bool capturing = captures((cudaStream_t)stream);
     FarConePlan& fc = D.fc[precision_ == PREC_MIXED];
-    if (!fc.ready && !fc.refused && !capturing)
+    if (!fc.ready && !fc.refused && !capturing && !captures(cudaStreamLegacy))
     {
         IFGF_CUDA(cudaSetDevice(device_));
         FarConeBuild b = far_cone_build(D, lv_);
         b.mixed = precision_ == PREC_MIXED;
+        // nor may its allocations end another thread's capture
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        IFGF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        struct Restore
+        {
+            cudaStreamCaptureMode mode;
+            ~Restore() { cudaThreadExchangeStreamCaptureMode(&mode); }
+        } restore{mode};
         build_far_cones(b, fc);
     }
     if (!fc.ready)
