@@ -2258,17 +2258,22 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
             }
             if constexpr (!MIXED && N0 > 0)
             {
-                ua.rch = ups64_rch<N0, N1, N2>(LL.fe_pad);
-                const size_t sm = ups64_smem<N0, N1, N2>(m.P_hi, ua.rch, LL.fe_pad);
-                if (LL.fe_pad > 0 && sm <= UP_STAGED_SMEM_MAX)
-                {
-                    auto kern = upward_staged64_kernel<KIND, N0, N1, N2>;
+                auto stage = [&](auto threads) {
+                    constexpr int TH = decltype(threads)::value;
+                    ua.rch = ups64_rch<N0, N1, N2>(LL.fe_pad, TH);
+                    const size_t sm = ups64_smem<N0, N1, N2>(m.P_hi, ua.rch, LL.fe_pad);
+                    if (LL.fe_pad <= 0 || sm > UP_STAGED_SMEM_MAX)
+                        return false;
+                    auto kern = upward_staged64_kernel<KIND, N0, N1, N2, TH>;
                     if (sm > 48 * 1024)
                         IFGF_CHECK(cudaFuncSetAttribute(
                             kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                    kern<<<LL.n_up, ups64_threads(N0 * N1 * N2), sm, st>>>(ua);
-                    staged = true;
-                }
+                    kern<<<LL.n_up, TH, sm, st>>>(ua);
+                    return true;
+                };
+                constexpr int TH = ups64_threads(N0 * N1 * N2);
+                staged = (LL.n_up <= UPS64_FEW && stage(std::integral_constant<int, 256>{})) ||
+                         stage(std::integral_constant<int, TH>{});
             }
             if constexpr (MIXED && N0 > 0 && (N0 * N1 * N2) % 2 == 0)
                 if (!staged)

@@ -93,10 +93,10 @@ __host__ __device__ constexpr int ups64_stride(int p_lo) { return p_lo | 1; }
 // Runs staged at a time: about 16 KB of blocks, at least four runs (rows
 // average a handful; a run has about ten groups of entries at p = 8 and some
 // twenty-five at p = 12).
-template <int N0, int N1, int N2> int ups64_rch(int fe_pad)
+template <int N0, int N1, int N2> int ups64_rch(int fe_pad, int threads)
 {
-    constexpr int fit0 = 16 * 1024 / (ups64_stride(N0 * N1 * N2) * (int)sizeof(double2));
-    constexpr int fit = fit0 > 4 ? fit0 : 4;
+    constexpr int per = ups64_stride(N0 * N1 * N2) * (int)sizeof(double2);
+    const int fit = std::max(4, (threads > 128 ? 48 : 16) * 1024 / per);
     return fe_pad < fit ? fe_pad : fit;
 }
 template <int N0, int N1, int N2> size_t ups64_smem(int P_hi, int rch, int fe_pad)
@@ -104,6 +104,13 @@ template <int N0, int N1, int N2> size_t ups64_smem(int P_hi, int rch, int fe_pa
     return ((size_t)P_hi + (size_t)rch * ups64_stride(N0 * N1 * N2)) * sizeof(double2) +
            ((size_t)16 * (fe_pad + 1) + 16) * sizeof(int);
 }
+
+// Levels of few cones, which leave SMs idle or short of warps, take 256 threads
+// per cone and stage three times the runs, where those CTAs (two per SM) all
+// reside at once: measured (ms) 264 cones 0.029 instead of 0.056, 192 cones
+// 0.031 instead of 0.068, but 663 cones 0.069 and 0.067, 917 cones 0.060 and
+// 0.051.
+constexpr int UPS64_FEW = 2 * 148;
 
 // Entries evaluated together per thread (sharing every coefficient load);
 // CTAs per SM give every thread 128 registers.
@@ -125,13 +132,12 @@ constexpr int UPS64_R = 2;
 // 2 / 64 / 16 / 10 29.7, 2 / 96 / 24 / 6 32.9, 4 / 64 / 24 / 6 30.1,
 // 4 / 64 / 16 / 4 35.6, 4 / 32 / 8 / 12 35.5: warps in flight are worth more
 // than fewer loads.
-template <int KIND, int N0, int N1, int N2>
-__global__ void __launch_bounds__(ups64_threads(N0* N1* N2), 512 / ups64_threads(N0 * N1 * N2))
+template <int KIND, int N0, int N1, int N2, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
     upward_staged64_kernel(const __grid_constant__ UpArgs a)
 {
     constexpr int R = UPS64_R;
     constexpr int P_LO = N0 * N1 * N2;
-    constexpr int THREADS = ups64_threads(P_LO);
     constexpr int BS = ups64_stride(P_LO);
     constexpr int SUB = UPGEO_RUN / R; // work items per table group
     constexpr bool REAL = KIND == K_LAPLACE;
