@@ -169,7 +169,7 @@ struct Layout
         pairs = b.leaf_off->back();
         // places at most: every cone with pairs wastes less than a tile
         most = (pairs + (FAR_TILE - 1) * std::min(n_fine, pairs) + 31) / 32 * 32;
-        fits = pairs > 0 && n_fine > 0 && most < (1ll << 31) - 1;
+        fits = pairs > 0 && n_fine > 0 && most < (1ll << 31) - 1 && n_fine < (1ll << 31) - 2;
         if (!fits)
             return;
         cub::DeviceScan::ExclusiveSum(nullptr, scan_b, (int*)nullptr, (int*)nullptr,
@@ -199,8 +199,17 @@ struct Layout
 void reserve_far_cones(const FarConeBuild& b, FarConePlan& plan)
 {
     const Layout at(b);
-    if (at.fits && at.bytes <= FAR_CONES_RESERVE)
+    if (!at.fits || at.bytes > FAR_CONES_RESERVE)
+        return;
+    try
+    {
         plan.mem.alloc(at.bytes);
+    }
+    catch (const Error&)
+    {
+        // an operator that just fits the device does without; the build tries
+        // again
+    }
 }
 
 void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
