@@ -85,10 +85,10 @@ inline KParams make_kparams(double kr, double ki, int dx)
 // ---------------------------------------------------------------------------
 // FP64 distance, phase and damping of the kernels.  With the library's square
 // root, division and sincos a Helmholtz (source, node) pair took about 150
-// instructions, 55 of them on the FP64 pipe; the forms below take about 75
-// and 42 and are at least as accurate (the phase k d is never rounded: its
-// reduction is exact through FMA; sums of 400 terms at k d <= 200 against
-// extended precision: 4.1e-15 relative, 4.9e-15 with the library's).
+// instructions, 55 of them on the FP64 pipe; the forms below take about 77
+// and 44.  The phase k d is never rounded: its reduction is exact through FMA.
+// tests/test_kernel_values.py holds single values to bounds derived from the
+// roundings (5.5 units for 1 / d); the library's rounded k d misses the phase's.
 // ---------------------------------------------------------------------------
 struct DistInv
 {
@@ -101,9 +101,14 @@ __device__ __forceinline__ bool tiny_square(double d2)
     return (unsigned)__double2hiint(d2) < 0x00100000u;
 }
 
-// The hardware's reciprocal-square-root estimate (about 20 bits), one step of
-// Halley's third-order iteration y (1 + e / 2 + 3 e^2 / 8), e = 1 - x y^2
-// (residual 5 e^3 / 16, below 2^-54), and one Newton correction of the root.
+// Root and reciprocal root together by Goldschmidt's coupled iteration with a
+// residual correction (P. Markstein, "Software division and square root using
+// Goldschmidt's algorithms", 6th Conference on Real Numbers and Computers,
+// 2004).  From the PTX estimate y of 1 / sqrt(x) (about 20 bits), g = x y and
+// h = y / 2 approach sqrt(x) and 1 / (2 sqrt(x)) with one relative error
+// r = 1/2 - g h in common; g + g r and h + h r square it.  The root then takes
+// its residual x - g^2, and the reciprocal i = 2 h its error 1 - i sqrt(x)
+// against that root.
 // Unless NORMAL (the caller has seen that d2 is a normal number), zero and
 // subnormal squares are scaled first; d2 = 0 gives d = 0, id = inf.
 template <bool NORMAL> __device__ __forceinline__ DistInv dist_inv(double d2)
@@ -113,13 +118,14 @@ template <bool NORMAL> __device__ __forceinline__ DistInv dist_inv(double d2)
     if (tiny)
         x = d2 * 0x1p200;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
+    double g = x * y, h = 0.5 * y;
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    const double i = h + h;
     DistInv q;
-    q.id = fma(fma(0.375, e, 0.5), e * y, y);
-    const double d0 = x * q.id;
-    // half the estimate (its exponent less one) is accurate enough here
-    const double h = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));
-    q.d = fma(fma(-d0, d0, x), h, d0);
+    q.d = fma(fma(-g, g, x), h, g);
+    q.id = fma(i, fma(-i, q.d, 1.0), i);
     if (tiny)
     {
         q.d = d2 == 0.0 ? 0.0 : q.d * 0x1p-100;
@@ -127,6 +133,23 @@ template <bool NORMAL> __device__ __forceinline__ DistInv dist_inv(double d2)
     }
     return q;
 }
+
+// The reciprocal alone by two steps of Newton's iteration y (3/2 - x y^2 / 2)
+template <bool NORMAL> __device__ __forceinline__ double dist_inverse(double d2)
+{
+    const bool tiny = !NORMAL && tiny_square(d2);
+    double x = d2, y;
+    if (tiny)
+        x = d2 * 0x1p200;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double c = 0.5 * x;
+    y *= fma(-(c * y), y, 1.5);
+    y = fma(y, fma(-(c * y), y, 0.5), y);
+    if (tiny)
+        y = d2 == 0.0 ? __longlong_as_double(0x7ff0000000000000ll) : y * 0x1p100;
+    return y;
+}
+
 // Polynomials through Chebyshev points (exact rational arithmetic, rounded):
 // sin(pi r / 2) / r in r^2 (the constant term as a hi + lo pair) and
 // (cos(pi r / 2) - 1) / r^2 in r^2 for |r| <= 1/2 (truncation 4e-18 and 1e-19
@@ -426,8 +449,8 @@ template <> struct Plugin<K_LAPLACE>
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP&)
     {
-        const DistInv q = dist_inv<KP::NORMAL>(dot3(x, x));
-        return {!KP::NORMAL && q.d == 0 ? 0.0 : q.id, 0.0};
+        const double d2 = dot3(x, x);
+        return {!KP::NORMAL && d2 == 0 ? 0.0 : dist_inverse<KP::NORMAL>(d2), 0.0};
     }
     __device__ static cplx<double> cf(const DistInv& q, const KParams&)
     {
@@ -442,8 +465,8 @@ template <> struct Plugin<K_LAPLACE>
     __device__ static void leaf_add(cplx<double>& s, const double* a, const double*,
                                     cplx<double> w, double, const KP&)
     {
-        const DistInv q = dist_inv<KP::NORMAL>(dot3(a, a));
-        s.re = fma(w.re, !KP::NORMAL && q.d == 0 ? 0.0 : q.id, s.re);
+        const double d2 = dot3(a, a);
+        s.re = fma(w.re, !KP::NORMAL && d2 == 0 ? 0.0 : dist_inverse<KP::NORMAL>(d2), s.re);
     }
 };
 

@@ -766,16 +766,22 @@ __global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_cons
                     }
                     if (!two)
                         w[1] = {0.0, 0.0};
+                    auto add = [&](cplx<double> wv, cplx<double> k) {
+                        if constexpr (KIND == K_LAPLACE) // real densities and values
+                            acc.re = fma(wv.re, k.re, acc.re);
+                        else
+                            cfma(acc, wv, k);
+                    };
                     if (!tiny)
                     {
 #pragma unroll
                         for (int r = 0; r < 2; r++)
-                            cfma(acc, w[r], P::kernel4pi(x[r], nv[r], kp));
+                            add(w[r], P::kernel4pi(x[r], nv[r], kp));
                     }
                     else
 #pragma unroll
                         for (int r = 0; r < 2; r++)
-                            cfma(acc, w[r], P::kernel4pi(x[r], nv[r], a.kp));
+                            add(w[r], P::kernel4pi(x[r], nv[r], a.kp));
                 }
             }
         }

@@ -1,0 +1,69 @@
+"""Single FP64 kernel values on the GPU (one source, one target each) against
+extended precision, in units of the rounding error, over the range of distances:
+from direct_eval, which takes any square of the distance, and from the matvec's
+near field, whose loop has seen that the squares are normal numbers."""
+import numpy as np
+import pytest
+
+import ifgf_b200 as G
+from ifgf_b200 import workloads as W
+
+U = 2.0 ** -53
+PI = np.longdouble("3.14159265358979323846264338327950288")
+
+
+def _values(op, y):
+    """(direct_eval, matvec) at the targets y for a source of density 1 at 0; eight
+    sources of density 0 around it make every target a near one."""
+    r = 0.6 * np.abs(y).max()
+    op.init(np.array([(0, 0, 0)] + [(a, b, c) for a in (-r, r) for b in (-r, r) for c in (-r, r)]).T, y)
+    w = np.zeros(9, dtype=np.float64 if isinstance(op, G.LaplaceIfgfOperator) else np.complex128)
+    w[0] = 1.0
+    return op.direct_eval(w, np.arange(y.shape[1])), op.mult(w)
+
+
+def _targets(m, seed):
+    y = W.sphere_points(m, seed=seed)
+    return y / np.linalg.norm(y, axis=0) * np.random.default_rng(seed).uniform(0.5, 2.0, m)
+
+
+def _distance(y):
+    return np.sqrt((y.astype(np.longdouble) ** 2).sum(0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1e-150, 1e-77, 1.0, 3e77, 1e150])
+def test_reciprocal_distance(scale):
+    y = _targets(4000, seed=1) * scale
+    ref = 1 / (4 * PI * _distance(y))
+    # three products and two sums of the square (half of 3 u), the reciprocal
+    # root to one unit in the last place (2 u), 1 / (4 pi) and its product (2 u)
+    for u in _values(G.LaplaceIfgfOperator(5000, 8), y):
+        assert np.max(np.abs(u / ref - 1)) <= 5.5 * U, float(np.max(np.abs(u / ref - 1)) / U)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1e-3, 1.0, 1e3])
+@pytest.mark.parametrize("kd", [1.0, 150.0, 600.0])
+def test_phase(scale, kd):
+    y = _targets(4000, seed=2) * scale
+    d = _distance(y)
+    k = kd / scale
+    ph = np.longdouble(k) * d
+    ref = (np.cos(ph) + 1j * np.sin(ph)) / (4 * PI * d)
+    # the modulus as above; sine and cosine to 3 u; the phase carries k times
+    # the distance's error (1.5 u of its square, 1 u of the root)
+    tol = U * (5.5 + 3 + 2.5 * ph.astype(np.float64))
+    for u in _values(G.HelmholtzIfgfOperator(k, 5000, 8), y):
+        assert np.all(np.abs(u / ref - 1) <= tol), float(np.max(np.abs(u / ref - 1) / tol))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kr", [0.5, 30.0, 300.0, -150.0])
+def test_damping(kr):
+    y = _targets(4000, seed=3)
+    d = _distance(y)
+    ref = np.exp(-np.longdouble(kr) * d) / (4 * PI * d)
+    tol = U * (5.5 + 3 + 2.5 * abs(kr) * d.astype(np.float64))
+    for u in _values(G.ModifiedHelmholtzIfgfOperator(complex(kr, 0.0), 5000, 8), y):
+        assert np.all(np.abs(u / ref - 1) <= tol), float(np.max(np.abs(u / ref - 1) / tol))
