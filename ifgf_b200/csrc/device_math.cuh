@@ -38,6 +38,7 @@ template <typename R> __device__ __forceinline__ void cfma(cplx<R>& acc, cplx<R>
 
 constexpr double INV4PI = 1.0 / (4.0 * 3.14159265358979323846);
 constexpr double DPI = 3.14159265358979323846;
+constexpr double INF64 = __builtin_huge_val();
 
 // Wavenumber and plug-in switches shared by all kernels of one operator.
 struct KParams
@@ -95,10 +96,11 @@ struct DistInv
     double d, id; // sqrt(d2), 1 / sqrt(d2)
 };
 
-// whether d2 >= 0 is zero or subnormal
-__device__ __forceinline__ bool tiny_square(double d2)
+// whether a square of a distance is anything but a normal number: zero or
+// subnormal, or beyond the range (infinity, NaN)
+__device__ __forceinline__ bool odd_square(double d2)
 {
-    return (unsigned)__double2hiint(d2) < 0x00100000u;
+    return (unsigned)(__double2hiint(d2) - 0x00100000) >= 0x7fe00000u;
 }
 
 // Root and reciprocal root together by Goldschmidt's coupled iteration with a
@@ -110,12 +112,13 @@ __device__ __forceinline__ bool tiny_square(double d2)
 // its residual x - g^2, and the reciprocal i = 2 h its error 1 - i sqrt(x)
 // against that root.
 // Unless NORMAL (the caller has seen that d2 is a normal number), zero and
-// subnormal squares are scaled first; d2 = 0 gives d = 0, id = inf.
+// subnormal squares are scaled first; d2 = 0 gives d = 0, id = inf, and
+// d2 = inf d = inf, id = 0.
 template <bool NORMAL> __device__ __forceinline__ DistInv dist_inv(double d2)
 {
-    const bool tiny = !NORMAL && tiny_square(d2);
+    const bool odd = !NORMAL && odd_square(d2);
     double x = d2, y;
-    if (tiny)
+    if (odd)
         x = d2 * 0x1p200;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     double g = x * y, h = 0.5 * y;
@@ -126,10 +129,11 @@ template <bool NORMAL> __device__ __forceinline__ DistInv dist_inv(double d2)
     DistInv q;
     q.d = fma(fma(-g, g, x), h, g);
     q.id = fma(i, fma(-i, q.d, 1.0), i);
-    if (tiny)
+    if (odd)
     {
-        q.d = d2 == 0.0 ? 0.0 : q.d * 0x1p-100;
-        q.id = d2 == 0.0 ? __longlong_as_double(0x7ff0000000000000ll) : q.id * 0x1p100;
+        const bool end = d2 == 0.0 || d2 == INF64;
+        q.d = end ? d2 : q.d * 0x1p-100;
+        q.id = d2 == 0.0 ? INF64 : d2 == INF64 ? 0.0 : q.id * 0x1p100;
     }
     return q;
 }
@@ -137,16 +141,16 @@ template <bool NORMAL> __device__ __forceinline__ DistInv dist_inv(double d2)
 // The reciprocal alone by two steps of Newton's iteration y (3/2 - x y^2 / 2)
 template <bool NORMAL> __device__ __forceinline__ double dist_inverse(double d2)
 {
-    const bool tiny = !NORMAL && tiny_square(d2);
+    const bool odd = !NORMAL && odd_square(d2);
     double x = d2, y;
-    if (tiny)
+    if (odd)
         x = d2 * 0x1p200;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double c = 0.5 * x;
     y *= fma(-(c * y), y, 1.5);
     y = fma(y, fma(-(c * y), y, 0.5), y);
-    if (tiny)
-        y = d2 == 0.0 ? __longlong_as_double(0x7ff0000000000000ll) : y * 0x1p100;
+    if (odd)
+        y = d2 == 0.0 ? INF64 : d2 == INF64 ? 0.0 : y * 0x1p100;
     return y;
 }
 

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(FAR_CONE_THREADS)
                              a.tz[t] - a.T.box_c[3 * box + 2]};
         const double r2 = fma(p[0], p[0], p[1] * p[1]), d2 = fma(p[2], p[2], r2);
         double x[3];
-        if (ct.y && !tiny_square(r2))
+        if (ct.y && !odd_square(r2) && d2 < INF64)
         {
             // angles relative to the cone's centre line, from the sines of
             // their differences

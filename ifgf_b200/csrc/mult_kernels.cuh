@@ -206,17 +206,16 @@ __global__ void __launch_bounds__(NODE_THREADS, 3) leaf_sample_kernel(LeafArgs a
             const double2 s3 = P::needs_normals ? s[ROWS - 1] : make_double2(0.0, 0.0);
             const double nv[3] = {s2.y, s3.x, s3.y};
             double av[NPT][3];
-            bool tiny = false;
+            bool odd = false;
 #pragma unroll
             for (int q = 0; q < NPT; q++)
             {
                 av[q][0] = s0.x - y[q][0];
                 av[q][1] = s0.y - y[q][1];
                 av[q][2] = s1.x - y[q][2];
-                tiny |= tiny_square(av[q][0] * av[q][0] + av[q][1] * av[q][1] +
-                                    av[q][2] * av[q][2]);
+                odd |= odd_square(dot3(av[q], av[q]));
             }
-            if (!tiny)
+            if (!odd)
             {
 #pragma unroll
                 for (int q = 0; q < NPT; q++)
@@ -750,7 +749,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_cons
                     const bool two = i + S < ccnt;
                     double x[2][3], nv[2][3];
                     cplx<double> w[2];
-                    bool tiny = false;
+                    bool odd = false;
 #pragma unroll
                     for (int r = 0; r < 2; r++)
                     {
@@ -762,7 +761,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_cons
                         x[r][2] = s1.x - y2;
                         w[r] = {s1.y, s2.x};
                         nv[r][0] = s2.y, nv[r][1] = s3.x, nv[r][2] = s3.y;
-                        tiny |= tiny_square(dot3(x[r], x[r]));
+                        odd |= odd_square(dot3(x[r], x[r]));
                     }
                     if (!two)
                         w[1] = {0.0, 0.0};
@@ -772,7 +771,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_cons
                         else
                             cfma(acc, wv, k);
                     };
-                    if (!tiny)
+                    if (!odd)
                     {
 #pragma unroll
                         for (int r = 0; r < 2; r++)
