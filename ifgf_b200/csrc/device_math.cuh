@@ -2,7 +2,9 @@
 // coordinates, cone lookups, Chebyshev evaluation and the six kernel plug-ins.
 #pragma once
 
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include <cuda_runtime.h>
 
@@ -53,7 +55,10 @@ struct KParams
     // FP64 phases and damping in the units their reductions use, as hi + lo
     // pairs: quarter turns 2 kr / pi and -2 ki / pi, octaves -kr / ln 2
     double qrh, qrl, qih, qil, erh, erl;
+    // odd_square's range of squares whose damping is a normal number
+    unsigned damp_range;
 };
+constexpr unsigned NORMAL_SQUARES = 0x7fe00000u;
 
 // a (bh + bl) as an unevaluated sum
 inline void scaled_pair(double a, double bh, double bl, double* h, double* l)
@@ -61,6 +66,9 @@ inline void scaled_pair(double a, double bh, double bl, double* h, double* l)
     *h = a * bh;
     *l = fma(a, bh, -*h) + a * bl;
 }
+
+// octaves of damping (or growth) that leave a normal number
+constexpr double DAMP_OCTAVES = 1020.0;
 
 inline KParams make_kparams(double kr, double ki, int dx)
 {
@@ -80,6 +88,15 @@ inline KParams make_kparams(double kr, double ki, int dx)
     p.trl = (float)(0.25 * p.qrh - (double)p.trh);
     p.tih = (float)(0.25 * p.qih);
     p.til = (float)(0.25 * p.qih - (double)p.tih);
+    p.damp_range = NORMAL_SQUARES;
+    if (p.erh != 0.0)
+    {
+        const double lim = DAMP_OCTAVES / std::fabs(p.erh), sq = lim * lim;
+        unsigned long long bits;
+        std::memcpy(&bits, &sq, sizeof bits);
+        const unsigned hi = (unsigned)(bits >> 32);
+        p.damp_range = hi > 0x00100000u ? std::min(hi - 0x00100000u, NORMAL_SQUARES) : 0u;
+    }
     return p;
 }
 
@@ -96,11 +113,11 @@ struct DistInv
     double d, id; // sqrt(d2), 1 / sqrt(d2)
 };
 
-// whether a square of a distance is anything but a normal number: zero or
-// subnormal, or beyond the range (infinity, NaN)
-__device__ __forceinline__ bool odd_square(double d2)
+// whether a square of a distance is anything but a normal number (zero or
+// subnormal, infinity, NaN), or one beyond `range`
+__device__ __forceinline__ bool odd_square(double d2, unsigned range = NORMAL_SQUARES)
 {
-    return (unsigned)(__double2hiint(d2) - 0x00100000) >= 0x7fe00000u;
+    return (unsigned)(__double2hiint(d2) - 0x00100000) >= range;
 }
 
 // Root and reciprocal root together by Goldschmidt's coupled iteration with a
@@ -203,7 +220,7 @@ struct PolyRegs
     __device__ __forceinline__ double exp2(int i) const { return e[i]; }
 };
 // KParams of a loop that keeps the coefficients in registers and has seen
-// that the squared distances are normal numbers
+// that the squared distances and the damping are normal numbers
 struct KParamsRegs : KParams
 {
     static constexpr bool NORMAL = true;
@@ -245,8 +262,8 @@ __device__ __forceinline__ cplx<double> quarter_turns(double qh, double ql, doub
 
 // e^{-kr d} as 2^t, t = (erh + erl) d: 2^f scaled through the exponent field.
 // Without branches (they would keep the compiler from interleaving a
-// thread's evaluations): beyond the normal range the result is infinity, or
-// zero (from 2^-1021 down).
+// thread's evaluations).  Unless NORMAL the scaling takes two products, the
+// second of which rounds to a subnormal number, zero or infinity.
 template <class KP> __device__ __forceinline__ double damping(const KP& p, double d)
 {
     const double m = fma(p.erh, d, ROUND_MAGIC);
@@ -258,10 +275,14 @@ template <class KP> __device__ __forceinline__ double damping(const KP& p, doubl
     for (int i = EXP2_N - 2; i >= 0; i--)
         e = fma(e, f, k.exp2(i));
     e = fma(e, f, 1.0);
+    if constexpr (KP::NORMAL)
+        return __hiloint2double(__double2hiint(e) + (n << 20), __double2loint(e));
     // m's high word is 0x43380000 (0x4337ffff) for 0 <= n (< 0) in 32 bits
-    const bool in = (unsigned)(n + 1021) <= 2044u && (unsigned)(mh - 0x4337ffff) <= 1u;
-    const int hi = in ? __double2hiint(e) + (n << 20) : (mh < 0x43380000 ? 0 : 0x7ff00000);
-    return __hiloint2double(hi, in ? __double2loint(e) : 0);
+    const bool in = (unsigned)(mh - 0x4337ffff) <= 1u;
+    const int t = in ? min(max(n, -1200), 1200) : (mh < 0x43380000 ? -1200 : 1200);
+    const int half = t >> 1;
+    return (in ? e : 1.0) * __hiloint2double((half + 1023) << 20, 0) *
+           __hiloint2double((t - half + 1023) << 20, 0);
 }
 
 // f e^{-k d} for complex k: f e^{-kr d} (cos(ki d), -sin(ki d))
@@ -432,7 +453,8 @@ __device__ __forceinline__ cplx<double> cheb_eval3(const double2* __restrict__ c
 //              dc = |y - xc|: the factor that depends on the node alone is
 //              applied once to the sum
 // kernel4pi and leaf_add take KParams, or KParamsRegs where the caller knows
-// that |x|^2 (|a|^2) is a normal number.
+// that |x|^2 (|a|^2) is a normal number, and the damping (of kernels that have
+// one: `damped`) over |x| (|a| - dc) too.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double dot3(const double* a, const double* b)
 {
@@ -449,6 +471,7 @@ template <int KIND> struct Plugin;
 // laplace_ifgf.hpp
 template <> struct Plugin<K_LAPLACE>
 {
+    static constexpr bool damped = false;
     static constexpr bool needs_normals = false;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP&)
@@ -477,6 +500,7 @@ template <> struct Plugin<K_LAPLACE>
 // helmholtz_ifgf.hpp (real k)
 template <> struct Plugin<K_HELMHOLTZ>
 {
+    static constexpr bool damped = false;
     static constexpr bool needs_normals = false;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
@@ -506,6 +530,7 @@ template <> struct Plugin<K_HELMHOLTZ>
 // modified_helmholtz_ifgf.hpp (complex k, kernel e^{-kd}/(4 pi d))
 template <> struct Plugin<K_MODHELMHOLTZ>
 {
+    static constexpr bool damped = true;
     static constexpr bool needs_normals = false;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
@@ -535,6 +560,7 @@ template <> struct Plugin<K_MODHELMHOLTZ>
 // grad_helmholtz_ifgf.hpp (complex k, derivative along dx, or plain if -1)
 template <> struct Plugin<K_GRADHELMHOLTZ>
 {
+    static constexpr bool damped = true;
     static constexpr bool needs_normals = false;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
@@ -578,6 +604,7 @@ template <> struct Plugin<K_GRADHELMHOLTZ>
 // double_layer_helmholtz_ifgf.hpp (complex k, source normals)
 template <> struct Plugin<K_DOUBLELAYER>
 {
+    static constexpr bool damped = true;
     static constexpr bool needs_normals = true;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double* n, const KP& p)
@@ -614,6 +641,7 @@ template <> struct Plugin<K_DOUBLELAYER>
 // e^{i kap d} / d^3 (nxy - i kap (d nxy + d^2)), nxy = -n . x
 template <> struct Plugin<K_COMBINEDFIELD>
 {
+    static constexpr bool damped = false;
     static constexpr bool needs_normals = true;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double* n, const KP& p)
@@ -655,6 +683,7 @@ template <> struct Plugin<K_COMBINEDFIELD>
 // e^{ik(r - r_p)}.
 template <> struct Plugin<K_HELMHOLTZ_DK>
 {
+    static constexpr bool damped = false;
     static constexpr bool needs_normals = false;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double*, const KP& p)
@@ -687,6 +716,7 @@ template <> struct Plugin<K_HELMHOLTZ_DK>
 // nxy = -n . x.  Centred factor and centre shift as for K_HELMHOLTZ_DK.
 template <> struct Plugin<K_COMBINEDFIELD_DK>
 {
+    static constexpr bool damped = false;
     static constexpr bool needs_normals = true;
     template <class KP>
     __device__ static cplx<double> kernel4pi(const double* x, const double* n, const KP& p)

@@ -151,6 +151,8 @@ __global__ void __launch_bounds__(NODE_THREADS, 3) leaf_sample_kernel(LeafArgs a
     const double xc[3] = {a.T.box_c[3 * box], a.T.box_c[3 * box + 1], a.T.box_c[3 * box + 2]};
     const double H = a.T.box_H[box];
     const KParamsRegs kp(a.kp);
+    // | |x - y| - |xc - y| | <= |x - xc| < H
+    const bool steep = P::damped && fabs(a.kp.erh) * H >= DAMP_OCTAVES;
     const int nt = blockDim.x;
     const int f = a.T.box_first[box], l = a.T.box_last[box];
     // a chunk's source of this thread; the first chunk's loads run ahead of
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(NODE_THREADS, 3) leaf_sample_kernel(LeafArgs a
             const double2 s3 = P::needs_normals ? s[ROWS - 1] : make_double2(0.0, 0.0);
             const double nv[3] = {s2.y, s3.x, s3.y};
             double av[NPT][3];
-            bool odd = false;
+            bool odd = steep;
 #pragma unroll
             for (int q = 0; q < NPT; q++)
             {
@@ -761,7 +763,8 @@ __global__ void __launch_bounds__(NEAR_THREADS, 3) near_kernel(const __grid_cons
                         x[r][2] = s1.x - y2;
                         w[r] = {s1.y, s2.x};
                         nv[r][0] = s2.y, nv[r][1] = s3.x, nv[r][2] = s3.y;
-                        odd |= odd_square(dot3(x[r], x[r]));
+                        odd |= odd_square(dot3(x[r], x[r]),
+                                          P::damped ? a.kp.damp_range : NORMAL_SQUARES);
                     }
                     if (!two)
                         w[1] = {0.0, 0.0};

@@ -8,6 +8,8 @@ import pytest
 import ifgf_b200 as G
 from ifgf_b200 import workloads as W
 
+from .helpers import KERNELS, densities_for, make_gpu_op
+
 U = 2.0 ** -53
 PI = np.longdouble("3.14159265358979323846264338327950288")
 
@@ -79,3 +81,30 @@ def test_squares_beyond_the_range():
     assert (ref == 0).any() and (ref > 0).any()
     for u in _values(G.LaplaceIfgfOperator(5000, 8), y):
         assert np.all(np.abs(u - ref) <= 5.5 * U * ref)
+
+
+@pytest.mark.gpu
+def test_damping_to_underflow():
+    """Values from e^{-200} down through the subnormal numbers to zero."""
+    y = _targets(4000, seed=5)
+    d = _distance(y)
+    ref = np.exp(-np.longdouble(400) * d) / (4 * PI * d)
+    tiny = np.longdouble(2) ** -1074
+    assert (ref > 2 ** -1000).any() and ((ref < 2 ** -1023) & (ref > 8 * tiny)).any()
+    # as test_damping, and up to four roundings to whole subnormal units
+    tol = U * (5.5 + 3 + 2.5 * 400 * d) * ref + 2 * tiny
+    for u in _values(G.ModifiedHelmholtzIfgfOperator(400 + 0j, 5000, 8), y):
+        assert np.all(np.abs(u - ref) <= tol), float(np.max(np.abs(u - ref) / tol))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["modified_helmholtz", "grad_helmholtz", "double_layer"])
+def test_leaf_with_steep_damping(name):
+    """Damping across a leaf of more than the normal range's octaves: the far
+    values underflow and stay finite on the way."""
+    src = W.sphere_points(300, seed=6)
+    op = make_gpu_op(name, leaf=500, order=8, dx=0, k=complex(380.0, 3.0))
+    tgt = 0.3 * W.sphere_points(200, seed=7) + np.array([[5.0], [0.0], [0.0]])
+    op.init(src, tgt, *((src,) if KERNELS[name][2] else ()))
+    assert op.stats()["target_leaf_far_evals"] > 0
+    assert np.all(op.mult(densities_for(name, 300)) == 0)
