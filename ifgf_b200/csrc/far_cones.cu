@@ -270,7 +270,8 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
                 host.data() + (at.trig - at.host));
     std::copy_n((const unsigned char*)level.data(), level.size() * sizeof(int2),
                 host.data() + (at.lev - at.host));
-    IFGF_CUDA(cudaMemcpy(m + at.host, host.data(), host.size(), cudaMemcpyHostToDevice));
+    const cudaStream_t st = b.stream;
+    IFGF_CUDA(cudaMemcpyAsync(m + at.host, host.data(), host.size(), cudaMemcpyHostToDevice, st));
     int* pos = (int*)(m + at.pos);
     int* tgt = (int*)(m + at.tgt);
     int* tile = (int*)(m + at.tile);
@@ -279,27 +280,29 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
     int* count = (int*)(m + at.val);
     int* off = (int*)(m + at.val + at.count_b);
     size_t scan_b = at.scan_b;
-    IFGF_CUDA(cudaMemsetAsync(count, 0, (n_fine + 1) * sizeof(int), nullptr));
-    IFGF_CUDA(cudaMemsetAsync(tgt, 0xff, at.meta - at.tgt, nullptr)); // and the tiles
-    lookup_kernel<<<1, 32>>>(b.lv_dev, L, (LookupF*)(m + at.lookup));
+    IFGF_CUDA(cudaMemsetAsync(count, 0, (n_fine + 1) * sizeof(int), st));
+    IFGF_CUDA(cudaMemsetAsync(tgt, 0xff, at.meta - at.tgt, st)); // and the tiles
+    lookup_kernel<<<1, 32, 0, st>>>(b.lv_dev, L, (LookupF*)(m + at.lookup));
     for (int l = 0; l < L; l++)
         if (lv[l].n_fine > 0)
-            meta_kernel<<<blocks_for(lv[l].n_fine), 256>>>(b.cone_box[l], b.cone_el[l],
-                                                           (int)lv[l].n_fine,
-                                                           meta + lv[l].fine_off);
+            meta_kernel<<<blocks_for(lv[l].n_fine), 256, 0, st>>>(b.cone_box[l], b.cone_el[l],
+                                                                  (int)lv[l].n_fine,
+                                                                  meta + lv[l].fine_off);
     const auto count_pairs = b.mixed ? count_kernel<true> : count_kernel<false>;
-    count_pairs<<<nl, THREADS>>>(b.lv_dev, b.T, b.tx, b.ty, b.tz, b.fmap, b.tl_first, b.tl_last,
-                                 b.far_off, b.far_src, leaf_off, pos, count, b.err, L);
-    pad_kernel<<<blocks_for(n_fine), 256>>>(count, (int)n_fine);
+    count_pairs<<<nl, THREADS, 0, st>>>(b.lv_dev, b.T, b.tx, b.ty, b.tz, b.fmap, b.tl_first,
+                                        b.tl_last, b.far_off, b.far_src, leaf_off, pos, count,
+                                        b.err, L);
+    pad_kernel<<<blocks_for(n_fine), 256, 0, st>>>(count, (int)n_fine);
     IFGF_CUDA(cub::DeviceScan::ExclusiveSum(m + at.val + 2 * at.count_b, scan_b, count, off,
-                                            (int)n_fine + 1));
-    tile_kernel<<<blocks_for(n_fine), 256>>>(off, (int)n_fine, tile);
-    int used = 0;
-    IFGF_CUDA(cudaMemcpy(&used, off + n_fine, sizeof(int), cudaMemcpyDeviceToHost));
-    // off becomes every cone's cursor
-    place_kernel<<<nl, THREADS>>>(b.tl_first, b.tl_last, b.far_off, leaf_off, pos, off, tgt);
+                                            (int)n_fine + 1, st));
+    tile_kernel<<<blocks_for(n_fine), 256, 0, st>>>(off, (int)n_fine, tile);
+    // every cone's entry of off becomes its cursor; the last one stays
+    place_kernel<<<nl, THREADS, 0, st>>>(b.tl_first, b.tl_last, b.far_off, leaf_off, pos, off,
+                                         tgt);
     IFGF_CUDA(cudaGetLastError());
-    IFGF_CUDA(cudaDeviceSynchronize());
+    int used = 0;
+    IFGF_CUDA(cudaMemcpyAsync(&used, off + n_fine, sizeof(int), cudaMemcpyDeviceToHost, st));
+    IFGF_CUDA(cudaStreamSynchronize(st));
     if (used == 0) // every pair outside its box's domain
     {
         plan.release();

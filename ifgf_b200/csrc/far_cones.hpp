@@ -40,6 +40,7 @@ struct FarConeBuild
     std::vector<const int*> cone_box, cone_el;
     unsigned long long* err;
     bool mixed = false; // lookups of the mixed pipeline
+    cudaStream_t stream = nullptr; // that the build runs on
 };
 
 // A plan is one allocation.  Small ones (up to FAR_CONES_RESERVE) get it with
@@ -50,7 +51,7 @@ void reserve_far_cones(const FarConeBuild& b, FarConePlan& plan);
 
 // Fills `plan`, or leaves it empty with `refused` set: no far pairs, 2^31
 // places or more, or more than a quarter of the free device memory (3.9e8
-// pairs take 12 ms).  Synchronises the device.
+// pairs take 12 ms).  Runs on the build's stream and waits for that one alone.
 void build_far_cones(const FarConeBuild& b, FarConePlan& plan);
 
 } // namespace ifgf

@@ -1840,23 +1840,22 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
     DeviceState& D = *dev_;
     if (!far_plan_on_ || D.n_tleaf == 0 || !far_cone_shape(lo_))
         return;
-    // the build allocates and runs on the legacy stream: not while `stream` is
-    // captured, nor while any stream is that the legacy one synchronises with
-    auto captures = [](cudaStream_t st) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) == cudaSuccess)
-            return cap != cudaStreamCaptureStatusNone;
+    // the build allocates and waits for `stream`: not while that is captured
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &cap) != cudaSuccess)
+    {
         cudaGetLastError();
-        return true;
-    };
-    const bool capturing = captures((cudaStream_t)stream);
+        cap = cudaStreamCaptureStatusActive; // the legacy stream beside a capture
+    }
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
     FarConePlan& fc = D.fc[precision_ == PREC_MIXED];
-    if (!fc.ready && !fc.refused && !capturing && !captures(cudaStreamLegacy))
+    if (!fc.ready && !fc.refused && !capturing)
     {
         IFGF_CUDA(cudaSetDevice(device_));
         FarConeBuild b = far_cone_build(D, lv_);
         b.mixed = precision_ == PREC_MIXED;
-        // nor may its allocations end another thread's capture
+        b.stream = (cudaStream_t)stream;
+        // its allocations must not end another thread's capture
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         IFGF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
         struct Restore
