@@ -23,6 +23,10 @@ static constexpr int ERR_INVALID = 1, ERR_CUDA = 2, ERR_STATE = 3, ERR_OOM = 4, 
             throw Error(ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_));           \
     } while (0)
 
+// Frees device memory that the library can do without (operators' far-cone
+// plans); false where there is none (operator.cu).
+bool give_back_device_memory();
+
 template <typename T> struct DevBuf
 {
     T* p = nullptr;
@@ -48,20 +52,30 @@ template <typename T> struct DevBuf
         return *this;
     }
     ~DevBuf() { release(); }
-    void alloc(size_t count)
+    // without giving anything back for it: for what can be done without
+    cudaError_t try_alloc(size_t count)
     {
         release();
         if (count == 0)
-            return;
-        cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
-        if (e != cudaSuccess)
+            return cudaSuccess;
+        const cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
+        if (e == cudaSuccess)
+            n = count;
+        else
         {
             cudaGetLastError();
             p = nullptr;
+        }
+        return e;
+    }
+    void alloc(size_t count)
+    {
+        cudaError_t e = try_alloc(count);
+        if (e == cudaErrorMemoryAllocation && give_back_device_memory())
+            e = try_alloc(count);
+        if (e != cudaSuccess)
             throw Error(ERR_OOM, "cudaMalloc(" + std::to_string(count * sizeof(T)) +
                                      " bytes) failed: " + cudaGetErrorString(e));
-        }
-        n = count;
     }
     void upload(const T* h, size_t count)
     {

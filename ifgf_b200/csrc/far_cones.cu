@@ -201,15 +201,8 @@ void reserve_far_cones(const FarConeBuild& b, FarConePlan& plan)
     const Layout at(b);
     if (!at.fits || at.bytes > FAR_CONES_RESERVE)
         return;
-    try
-    {
-        plan.mem.alloc(at.bytes);
-    }
-    catch (const Error&)
-    {
-        // an operator that just fits the device does without; the build tries
-        // again
-    }
+    // an operator that just fits the device does without; the build tries again
+    (void)plan.mem.try_alloc(at.bytes);
 }
 
 void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
@@ -252,12 +245,7 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
             return;
         }
     }
-    try
-    {
-        if (!plan.mem.p)
-            plan.mem.alloc(at.bytes);
-    }
-    catch (const Error&)
+    if (!plan.mem.p && plan.mem.try_alloc(at.bytes) != cudaSuccess)
     {
         plan.refused = true;
         return;

@@ -540,6 +540,19 @@ static std::vector<double> c2f_matrix(int ho, int lo, int f)
     return out;
 }
 
+// Every operator of the process (never destroyed: operators may outlive the
+// library's other statics).
+struct Operators
+{
+    std::mutex mutex;
+    std::vector<Operator*> all;
+};
+static Operators& operators()
+{
+    static Operators* o = new Operators;
+    return *o;
+}
+
 Operator::Operator(int kind, double k_re, double k_im, int64_t leaf_size, int64_t order,
                    int64_t n_elem, double tol)
     : kind_(kind), kr_(k_re), ki_(k_im), tol_(tol), leaf_(leaf_size), order0_((int)order)
@@ -560,9 +573,43 @@ Operator::Operator(int kind, double k_re, double k_im, int64_t leaf_size, int64_
     for (int i = 0; i < 3; i++)
         base_order_[i] = (int)order;
     dev_.reset(new DeviceState());
+    std::lock_guard<std::mutex> lock(operators().mutex);
+    operators().all.push_back(this);
 }
 
-Operator::~Operator() = default;
+Operator::~Operator()
+{
+    std::lock_guard<std::mutex> lock(operators().mutex);
+    auto& all = operators().all;
+    all.erase(std::find(all.begin(), all.end(), this));
+}
+
+bool Operator::give_back_plans(int device)
+{
+    std::unique_lock<std::mutex> lock(plans_, std::try_to_lock);
+    if (!lock || device_ != device)
+        return false;
+    bool any = false;
+    for (FarConePlan& fc : dev_->fc)
+        if (fc.mem.p && !fc.captured)
+        {
+            fc.release(); // waits for the matvecs under way
+            any = true;
+        }
+    return any;
+}
+
+bool give_back_device_memory()
+{
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess)
+        return false;
+    std::lock_guard<std::mutex> lock(operators().mutex);
+    bool any = false;
+    for (Operator* op : operators().all)
+        any = op->give_back_plans(device) || any;
+    return any;
+}
 
 void Operator::set_dx(int dx)
 {
@@ -1166,7 +1213,10 @@ void Operator::setup_device(const double* normals)
     D.dgeo32_ptr.clear();
     D.dgeo_ready = false;
     // the device this operator's tables live on
-    IFGF_CUDA(cudaGetDevice(&device_));
+    {
+        std::lock_guard<std::mutex> lock(plans_);
+        IFGF_CUDA(cudaGetDevice(&device_));
+    }
     const Tree& S = plan_.src;
     const Tree& Tt = plan_.tgt;
     const int L = S.num_levels();
@@ -1290,8 +1340,11 @@ void Operator::setup_device(const double* normals)
     D.fp_slot.release();
     D.fp_nchunk = 0;
     D.fp_ready = false;
-    for (FarConePlan& fc : D.fc)
-        fc.release();
+    {
+        std::lock_guard<std::mutex> lock(plans_);
+        for (FarConePlan& fc : D.fc)
+            fc.release();
+    }
     phase("target_leaf_lists");
     // ---- active cones (octree.hpp:351-816) on the GPU ----
     int64_t fmap_total = 0;
@@ -1624,7 +1677,10 @@ void Operator::setup_device(const double* normals)
     if (D.c2f_smem > 220 * 1024)
         throw Error(ERR_INVALID, "interpolation order too high for the coarse-to-fine kernel");
     if (precision_ == PREC_FP64 && far_plan_on_ && far_cone_shape(lo_))
+    {
+        std::lock_guard<std::mutex> lock(plans_);
         reserve_far_cones(far_cone_build(D, lv_), D.fc[0]);
+    }
     phase("buffers");
 }
 
@@ -1829,6 +1885,7 @@ void Operator::set_far_plan(bool on)
         D.fp_ready = false;
         // a captured graph may still read a far-cone plan: kept until the
         // next init
+        std::lock_guard<std::mutex> lock(plans_);
         for (FarConePlan& fc : D.fc)
             if (!fc.captured)
                 fc.release();
@@ -2384,13 +2441,16 @@ void Operator::launch_mult(const void* d_w, void* d_u, void* stream, bool timed,
     }
     MultPtrs m;
     fill_mult_ptrs(m, vkind >= 0);
-    ensure_far_cones(m, stream);
     EventHooks log(D, st);
     const bool on = profiling_ || timed;
     int launches = 0;
-    IFGF_DISPATCH(vkind >= 0 ? vkind : kind_,
-                  launches = launch_mult_kernels<KK>(m, d_w, d_u, is_real(), st,
-                                                     on ? &log : nullptr));
+    {
+        std::lock_guard<std::mutex> lock(plans_);
+        ensure_far_cones(m, stream);
+        IFGF_DISPATCH(vkind >= 0 ? vkind : kind_,
+                      launches = launch_mult_kernels<KK>(m, d_w, d_u, is_real(), st,
+                                                         on ? &log : nullptr));
+    }
     launches_per_mult_ = launches;
     if (on && log.n > 0)
         finish_profile(log, 1);
@@ -3078,10 +3138,12 @@ std::string Operator::stats_json() const
       << (dev_->fp_group.n * sizeof(FarGroup) + dev_->fp_rec.n * sizeof(FarPlanRec) +
           dev_->fp_slot.n * sizeof(int) + dev_->fp_chunk.n * sizeof(FarChunk))
       << ",\"slots_per_group\":" << dev_->fp_nslot << ",\"overflow_share_at_few_slots\":" << dev_->fp_ovf_few << ",\"build_ms\":" << dev_->fp_ms << "}";
+    std::unique_lock<std::mutex> lock(plans_);
     const FarConePlan& fc = dev_->fc[precision_ == PREC_MIXED];
     o << ",\"far_cones\":{\"built\":" << (fc.ready ? 1 : 0) << ",\"pairs\":" << fc.pairs
       << ",\"places\":" << fc.places << ",\"bytes\":" << fc.mem.n << ",\"build_ms\":" << fc.ms
       << "}";
+    lock.unlock();
     o << ",\"upward_images_bytes\":[";
     for (int l = 0; l < (int)lv_.size(); l++)
         o << (l ? "," : "") << (l < (int)dev_->tc_img.size() ? dev_->tc_img[l].n : 0);

@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -105,6 +106,9 @@ class Operator
     void set_far_plan(bool on);
     bool far_plan() const { return far_plan_on_; }
     int upward_path() const { return up_path_; }
+    // frees the far-cone plans that no capture holds, unless a matvec is being
+    // enqueued; whether there were any.  For any thread.
+    bool give_back_plans(int device);
     // throws IFGF_ERR_TIMEOUT when a tensor-core kernel's bounded wait gave up
     void check_device_status();
 
@@ -172,6 +176,9 @@ class Operator
     int lo_[3], hi_[3];
     int fct_[3];
     std::unique_ptr<DeviceState> dev_;
+    // held while the far-cone plans change or a matvec that reads one is
+    // enqueued; no DevBuf::alloc under it (that may ask for the plans)
+    mutable std::mutex plans_;
     // init inputs in the caller's order, kept for the adjoint operators
     std::vector<double> src_pts_, tgt_pts_, normals_;
     std::function<bool(double)> cutoff_;

@@ -54,3 +54,56 @@ def test_first_call_while_another_thread_captures(precision):
     assert rel2(ua.cpu().numpy(), ub.cpu().numpy()) <= 1e-12
     assert np.isfinite(ua.abs().sum().item())
     del graph
+
+
+def _free():
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _hold_all_but(n_bytes):
+    """A tensor that leaves about n_bytes of the device's memory."""
+    import torch
+
+    return torch.empty(_free() - n_bytes, dtype=torch.uint8, device="cuda")
+
+
+def _op(n, pts):
+    g = make_gpu_op("helmholtz", leaf=100, order=8)
+    g.init(pts, pts)
+    g.set_precision("mixed")
+    g.set_upward_path("ffma")
+    return g
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("same", [True, False])
+def test_plans_give_way_to_other_allocations(same):
+    """A batch whose planes find no room beside a plan -- the operator's own or
+    another operator's -- gets the plan's memory; later matvecs go on without or
+    build it again."""
+    n, rhs = 100000, 4
+    pts = W.sphere_points(n, seed=0)
+    w = np.stack([W.densities(n, seed=i) for i in range(rhs)])
+    a = _op(n, pts)
+    b = a if same else _op(n, pts)
+    ref = a.mult(w[0])
+    plan = a.stats()["far_cones"]["bytes"]
+    assert plan > 100 << 20
+    # what a batch takes: of an operator of its own
+    twin = _op(n, pts)
+    before = _free()
+    twin.mult_batch(w)
+    need = before - _free()
+    del twin
+    # (the staging buffers of host calls are a few MB of it)
+    held = _hold_all_but(need - plan // 2)
+    u = b.mult_batch(w)
+    assert a.stats()["far_cones"]["bytes"] == 0
+    del held
+    _free()
+    assert rel2(u[0], ref) <= 1e-6
+    assert rel2(a.mult(w[0]), ref) <= 1e-6
