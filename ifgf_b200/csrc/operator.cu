@@ -2653,6 +2653,7 @@ int Operator::ensure_batch_planes(int64_t want)
     if (D.b_planes >= planes && D.b_cv == D.cvals.n && D.b_fc == D.fcoef.n && D.b_ns == n_src() &&
         D.b_nt == n_tgt())
         return std::min(planes, D.b_planes);
+    D.b_planes = 0; // until all of them are there
     D.bw.alloc((size_t)planes * n_src());
     D.bcv.alloc((size_t)planes * D.cvals.n);
     D.bfc.alloc((size_t)planes * D.fcoef.n);
@@ -2857,6 +2858,7 @@ void Operator::mult_wavenumbers_device(const double* k, int64_t nk, const void* 
                  D.kp_host[i].dx == kps[i].dx;
     if (!same_k)
     {
+        D.kp_host.clear(); // until both tables are there
         if (D.kp_plane.n < kps.size())
             D.kp_plane.alloc(kps.size());
         if (D.kp_row.n < rows.size())

@@ -5,6 +5,7 @@ import threading
 import numpy as np
 import pytest
 
+from ifgf_b200 import IfgfError
 from ifgf_b200 import workloads as W
 
 from .helpers import make_gpu_op, rel2
@@ -107,3 +108,19 @@ def test_plans_give_way_to_other_allocations(same):
     _free()
     assert rel2(u[0], ref) <= 1e-6
     assert rel2(a.mult(w[0]), ref) <= 1e-6
+
+
+@pytest.mark.gpu
+def test_batch_after_one_that_found_no_memory():
+    n = 20000
+    pts = W.sphere_points(n, seed=0)
+    w = np.stack([W.densities(n, seed=i) for i in range(64)])
+    a = _op(n, pts)
+    a.set_far_plan(False)
+    ref = a.mult_batch(w[:2])
+    held = _hold_all_but(64 << 20)
+    with pytest.raises(IfgfError, match="out of memory"):
+        a.mult_batch(w)
+    del held
+    _free()
+    assert rel2(a.mult_batch(w[:2]), ref) <= 1e-6
