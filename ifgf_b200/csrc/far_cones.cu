@@ -15,6 +15,7 @@ void FarConePlan::release()
     p = FarConePtrs();
     pairs = places = 0;
     ready = refused = captured = false;
+    wait = 0;
 }
 
 namespace
@@ -241,13 +242,13 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
         IFGF_CUDA(cudaMemGetInfo(&free_b, &total_b));
         if (at.bytes > free_b / 4)
         {
-            plan.refused = true;
+            plan.wait = FAR_CONES_RETRY;
             return;
         }
     }
     if (!plan.mem.p && plan.mem.try_alloc(at.bytes) != cudaSuccess)
     {
-        plan.refused = true;
+        plan.wait = FAR_CONES_RETRY;
         return;
     }
     unsigned char* m = plan.mem.p;

@@ -17,7 +17,8 @@ struct FarConePlan
     long long pairs = 0, places = 0;
     double ms = 0;
     bool ready = false;
-    bool refused = false;  // not built for its size or for want of memory
+    bool refused = false;  // nothing to build, or too many places
+    int wait = 0;          // matvecs until another attempt, after want of memory
     bool captured = false; // a stream capture holds its addresses
     void release();
 };
@@ -49,9 +50,13 @@ struct FarConeBuild
 constexpr size_t FAR_CONES_RESERVE = size_t(64) << 20;
 void reserve_far_cones(const FarConeBuild& b, FarConePlan& plan);
 
-// Fills `plan`, or leaves it empty with `refused` set: no far pairs, 2^31
-// places or more, or more than a quarter of the free device memory (3.9e8
-// pairs take 12 ms).  Runs on the build's stream and waits for that one alone.
+// Without memory a plan is tried again after this many matvecs (asking for
+// the free memory takes some tens of microseconds).
+constexpr int FAR_CONES_RETRY = 16;
+
+// Fills `plan`, or leaves it empty: with `refused` set for no far pairs or 2^31
+// places or more, with `wait` set where it would take more than a quarter of
+// the free device memory or finds none (3.9e8 pairs take 12 ms).  Runs on the build's stream and waits for that one alone.
 void build_far_cones(const FarConeBuild& b, FarConePlan& plan);
 
 } // namespace ifgf

@@ -594,6 +594,7 @@ bool Operator::give_back_plans(int device)
         if (fc.mem.p && !fc.captured)
         {
             fc.release(); // waits for the matvecs under way
+            fc.wait = FAR_CONES_RETRY;
             any = true;
         }
     return any;
@@ -1906,7 +1907,7 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
     }
     const bool capturing = cap != cudaStreamCaptureStatusNone;
     FarConePlan& fc = D.fc[precision_ == PREC_MIXED];
-    if (!fc.ready && !fc.refused && !capturing)
+    if (!fc.ready && !fc.refused && !capturing && (fc.wait == 0 || --fc.wait == 0))
     {
         IFGF_CUDA(cudaSetDevice(device_));
         FarConeBuild b = far_cone_build(D, lv_);
@@ -3144,7 +3145,7 @@ std::string Operator::stats_json() const
     const FarConePlan& fc = dev_->fc[precision_ == PREC_MIXED];
     o << ",\"far_cones\":{\"built\":" << (fc.ready ? 1 : 0) << ",\"pairs\":" << fc.pairs
       << ",\"places\":" << fc.places << ",\"bytes\":" << fc.mem.n << ",\"build_ms\":" << fc.ms
-      << "}";
+      << ",\"refused\":" << (fc.refused || fc.wait > 0 ? 1 : 0) << "}";
     lock.unlock();
     o << ",\"upward_images_bytes\":[";
     for (int l = 0; l < (int)lv_.size(); l++)

@@ -124,3 +124,37 @@ def test_batch_after_one_that_found_no_memory():
     del held
     _free()
     assert rel2(a.mult_batch(w[:2]), ref) <= 1e-6
+
+
+@pytest.mark.gpu
+def test_plan_refused_for_want_of_memory_is_tried_again():
+    import torch
+
+    n = 50000
+    pts = W.sphere_points(n, seed=0)
+    w = torch.from_numpy(W.densities(n, seed=1)).cuda()
+    g = make_gpu_op("helmholtz", leaf=100, order=8)
+    g.init(pts, pts)
+    us = []
+
+    def mult():
+        us.append(torch.empty_like(w))
+        g.mult_device(w.data_ptr(), us[-1].data_ptr())
+        torch.cuda.synchronize()
+        return g.stats()["far_cones"]
+
+    us_room = torch.empty(32, n, dtype=w.dtype, device="cuda")  # for the results
+    held = _hold_all_but(64 << 20)
+    del us_room
+    st = mult()
+    assert st["built"] == 0 and st["refused"] == 1
+    del held
+    _free()
+    calls = 0
+    while not st["built"]:
+        st = mult()
+        calls += 1
+        assert calls <= 16
+    assert st["refused"] == 0
+    for u in us[1:]:
+        assert rel2(u.cpu().numpy(), us[0].cpu().numpy()) <= 1e-12
