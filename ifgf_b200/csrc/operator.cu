@@ -1913,6 +1913,10 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
         FarConeBuild b = far_cone_build(D, lv_);
         b.mixed = precision_ == PREC_MIXED;
         b.stream = (cudaStream_t)stream;
+        // what init reserved for an FP64 plan that was not built (a larger one)
+        FarConePlan& fp64 = D.fc[PREC_FP64];
+        if (b.mixed && !fc.mem.p && !fp64.ready)
+            fc.mem = std::move(fp64.mem);
         // its allocations must not end another thread's capture
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         IFGF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));

@@ -158,3 +158,23 @@ def test_plan_refused_for_want_of_memory_is_tried_again():
     assert st["refused"] == 0
     for u in us[1:]:
         assert rel2(u.cpu().numpy(), us[0].cpu().numpy()) <= 1e-12
+
+
+@pytest.mark.gpu
+def test_mixed_plan_takes_the_unused_reservation():
+    n = 4000
+    pts = W.sphere_points(n, seed=0)
+    w = W.densities(n, seed=1)
+    g = make_gpu_op("helmholtz", leaf=50, order=8)
+    g.init(pts, pts)
+    assert g.stats()["far_cones"]["bytes"] > 0  # with init's buffers
+    g.set_precision("mixed")
+    um = g.mult(w)
+    assert g.stats()["far_cones"]["built"] == 1
+    g.set_precision("fp64")
+    assert g.stats()["far_cones"]["bytes"] == 0
+    u = g.mult(w)
+    assert g.stats()["far_cones"]["built"] == 1
+    g.set_precision("mixed")
+    assert np.array_equal(g.mult(w), um)
+    assert rel2(um, u) <= 2e-5
