@@ -382,10 +382,11 @@ __global__ void __launch_bounds__(THREADS)
     }
 }
 
-void launch_far_gather(const MultPtrs& m, void* d_u, bool real, cudaStream_t st)
+void launch_far_gather(const MultPtrs& m, const FarConePtrs& fc, void* d_u, bool real,
+                       cudaStream_t st)
 {
     const auto kern = m.mixed ? far_gather_kernel<float2> : far_gather_kernel<double2>;
-    kern<<<m.n_tleaf, THREADS, 0, st>>>(m.fc, m.tl_first, m.tl_last, m.tl_far_off, m.unear,
+    kern<<<m.n_tleaf, THREADS, 0, st>>>(fc, m.tl_first, m.tl_last, m.tl_far_off, m.unear,
                                         m.tgt_perm, (double*)d_u, real ? 1 : 0);
 }
 

@@ -15,7 +15,7 @@ struct FarConePlan
     DevBuf<unsigned char> mem; // everything `p` points to
     FarConePtrs p;
     long long pairs = 0, places = 0;
-    double ms = 0;
+    double ms = 0; // of the build, the kernels enqueued before it included
     bool ready = false;
     bool refused = false;  // nothing to build, or too many places
     int wait = 0;          // matvecs until another attempt, after want of memory

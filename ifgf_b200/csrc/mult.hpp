@@ -2,6 +2,8 @@
 // instantiated once per kernel plug-in in kernels_k<KIND>.cu).
 #pragma once
 
+#include <functional>
+
 #include <cuda_runtime.h>
 
 #include "common.hpp"
@@ -179,14 +181,18 @@ struct MultPtrs
     // the upward-kernel autotuner's per-level choice for single-plane
     // matvecs (host array of L: 1 tensor cores, 0 FFMA, -1 none yet)
     const signed char* up_choice = nullptr;
-    // far-cone plan of the far field (null: the
-    // far kernel looks up every pair's cone)
+    // far-cone plan of the far field (null: the far kernel looks up every
+    // pair's cone), or what builds it: called when the kernels before the far
+    // field are enqueued, so that the build's allocation and host work (some
+    // 0.4 ms) overlap theirs
     FarConePtrs fc;
+    const std::function<FarConePtrs()>* build_fc = nullptr;
 };
 
 // Sums of a far-cone plan's values per target, plus the near sums, into the
 // caller's result (far_cones.cu).
-void launch_far_gather(const MultPtrs& m, void* d_u, bool real, cudaStream_t st);
+void launch_far_gather(const MultPtrs& m, const FarConePtrs& fc, void* d_u, bool real,
+                       cudaStream_t st);
 
 struct C2FArgs
 {

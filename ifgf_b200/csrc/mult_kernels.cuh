@@ -2351,18 +2351,19 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
     }
     if (m.n_tleaf > 0)
     {
+        const FarConePtrs fc = N0 > 0 && m.build_fc ? (*m.build_fc)() : m.fc;
         if (hk)
             hk->begin(PROF_EVAL);
         bool by_cone = false;
         if constexpr (N0 > 0)
-            if (m.fc.tile_cone)
+            if (fc.tile_cone)
             {
-                const FarConeArgs fa{m.fc, m.lv_dev, m.T, m.tx, m.ty, m.tz, m.fcoef, m.kp};
+                const FarConeArgs fa{fc, m.lv_dev, m.T, m.tx, m.ty, m.tz, m.fcoef, m.kp};
                 // groups of 32 places per CTA
                 constexpr int PER = FAR_CONE_THREADS / 32 * (MIXED ? FAR_CONE_PER : 1);
                 const auto kern = MIXED ? far_cone_mixed_kernel<KIND, N0, N1, N2>
                                         : far_cone_kernel<KIND, N0, N1, N2>;
-                kern<<<(unsigned)((m.fc.n_groups - 1) / PER + 1), FAR_CONE_THREADS, 0, st>>>(fa);
+                kern<<<(unsigned)((fc.n_groups - 1) / PER + 1), FAR_CONE_THREADS, 0, st>>>(fa);
                 IFGF_CHECK_LAUNCH();
                 launches++;
                 by_cone = true;
@@ -2371,7 +2372,7 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
         if (overlap)
             IFGF_CHECK(cudaStreamWaitEvent(st, m.ev_join, 0));
         if (by_cone)
-            launch_far_gather(m, d_u, real, st);
+            launch_far_gather(m, fc, d_u, real, st);
         else if (MIXED)
             target_eval_mixed_kernel<KIND, N0, N1, N2><<<m.n_tleaf, FAR_THREADS, 0, st>>>(ea);
         else

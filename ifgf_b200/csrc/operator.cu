@@ -1893,7 +1893,7 @@ void Operator::set_far_plan(bool on)
     }
 }
 
-void Operator::ensure_far_cones(MultPtrs& m, void* stream)
+void Operator::set_far_cones(MultPtrs& m, void* stream, std::function<FarConePtrs()>& build)
 {
     DeviceState& D = *dev_;
     if (!far_plan_on_ || D.n_tleaf == 0 || !far_cone_shape(lo_))
@@ -1907,8 +1907,15 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
     }
     const bool capturing = cap != cudaStreamCaptureStatusNone;
     FarConePlan& fc = D.fc[precision_ == PREC_MIXED];
-    if (!fc.ready && !fc.refused && !capturing && (fc.wait == 0 || --fc.wait == 0))
+    if (fc.ready)
     {
+        fc.captured |= capturing;
+        m.fc = fc.p;
+        return;
+    }
+    if (fc.refused || capturing || (fc.wait > 0 && --fc.wait > 0))
+        return;
+    build = [this, &D, &fc, stream] {
         IFGF_CUDA(cudaSetDevice(device_));
         FarConeBuild b = far_cone_build(D, lv_);
         b.mixed = precision_ == PREC_MIXED;
@@ -1926,11 +1933,9 @@ void Operator::ensure_far_cones(MultPtrs& m, void* stream)
             ~Restore() { cudaThreadExchangeStreamCaptureMode(&mode); }
         } restore{mode};
         build_far_cones(b, fc);
-    }
-    if (!fc.ready)
-        return;
-    fc.captured |= capturing;
-    m.fc = fc.p;
+        return fc.p;
+    };
+    m.build_fc = &build;
 }
 
 void Operator::ensure_far_plan()
@@ -2451,7 +2456,8 @@ void Operator::launch_mult(const void* d_w, void* d_u, void* stream, bool timed,
     int launches = 0;
     {
         std::lock_guard<std::mutex> lock(plans_);
-        ensure_far_cones(m, stream);
+        std::function<FarConePtrs()> build;
+        set_far_cones(m, stream, build);
         IFGF_DISPATCH(vkind >= 0 ? vkind : kind_,
                       launches = launch_mult_kernels<KK>(m, d_w, d_u, is_real(), st,
                                                          on ? &log : nullptr));

@@ -16,6 +16,7 @@ namespace ifgf
 {
 
 struct DeviceState;  // device buffers, defined in operator.cu
+struct FarConePtrs;  // far-cone plan as the kernels see it, mult.hpp
 struct MultPtrs;     // kernel launch view, defined in mult.hpp
 struct AdjointState; // operators and buffers of the adjoint, defined in operator.cu
 struct EventHooks;   // per-launch CUDA events, defined in operator.cu
@@ -141,9 +142,10 @@ class Operator
     // finds its cones itself (no plan memory)
     void ensure_far_plan();
     void set_batch_far(BatchPtrs& bp);
-    // far-cone plan of the single matvec in this precision (built on first
-    // use, once per init; not while `stream` is being captured)
-    void ensure_far_cones(MultPtrs& m, void* stream);
+    // far-cone plan of the single matvec in this precision: handed to the
+    // kernels through m, or `build`, which builds it (on first use, once per
+    // init; not while `stream` is being captured)
+    void set_far_cones(MultPtrs& m, void* stream, std::function<FarConePtrs()>& build);
     void ensure_upward_tuned(int planes, const BatchPtrs* bp, void* stream);
     // basis images of the tensor-core upward transfer (built on first use of
     // the mixed pipeline; their entry data is rewritten by set_wavenumber)
