@@ -1109,13 +1109,15 @@ __device__ __forceinline__ cplx<float> transfer_delta(float delta, float ratio, 
     return {e.re * ratio, e.im * ratio};
 }
 
-// FP32 coordinates: (s, theta, phi) from an FP32 difference vector
+// FP32 coordinates: (s, theta, phi) from an FP32 difference vector.  Roundings
+// are spelled out (the compiler could contract products and sums differently
+// in every kernel), so that all kernels get the same coordinates.
 __device__ __forceinline__ void cart_to_interp_f(float p0, float p1, float p2, float H, float* s)
 {
-    const float a = p0 * p0 + p1 * p1;
+    const float a = __fmaf_rn(p1, p1, __fmul_rn(p0, p0));
     s[2] = fminf(fmaxf(atan2f(p1, p0), -(float)DPI), (float)DPI);
     s[1] = fminf(fmaxf(atan2f(sqrtf(a), p2), 0.f), (float)DPI);
-    s[0] = H * rsqrtf(a + p2 * p2);
+    s[0] = __fmul_rn(H, rsqrtf(__fmaf_rn(p2, p2, a)));
 }
 
 
@@ -1143,8 +1145,7 @@ __device__ __forceinline__ void make_lookupf(const LevelGeom& G, LookupF& L)
 // Fine element of the point p in FP32 (-1 outside the domain) and its local
 // coordinates: with t = (s - lo) / h the element index is q = floor(t)
 // (clamped) and the local coordinate 2 (t - q) - 1, the same quantities as
-// (s - centre) / (h / 2).  Roundings are spelled out, so that every kernel that
-// looks a pair up gets the same coordinates.
+// (s - centre) / (h / 2), the same in every kernel (roundings spelled out).
 __device__ __forceinline__ int lookup_f(const LookupF& L, const double* p, double H, float* loc)
 {
     float sf[3];
