@@ -59,8 +59,8 @@ REF_BUDGET_S = 100.0
 # dram__bytes_read.sum + dram__bytes_write.sum
 # (profiles/launches_bench_1e6_mixed_batched.md)
 UPWARD_FFMA_DRAM_B = 19.3
-UPWARD_TC_DRAM_B = 22.2
-FAR_DRAM_B = 26.7
+UPWARD_TC_DRAM_B = 22.6
+FAR_DRAM_B = 26.8
 
 
 def parse():
@@ -571,7 +571,7 @@ def run_ours(a):
     # DRAM bytes per padded geometry-table entry and right-hand side, per
     # upward kernel, and per (target, far box) pair and right-hand side of
     # the far field: one ncu capture of dram__bytes_read.sum +
-    # dram__bytes_write.sum of this bench command at full size, summed over
+    # dram__bytes_write.sum of this bench's matvec at full size, summed over
     # the launches of each kernel and divided by the units they processed
     # (profiles/launches_bench_1e6_mixed_batched.md)
     bytes_per_unit = {"upward_ffma": UPWARD_FFMA_DRAM_B, "upward_tensor": UPWARD_TC_DRAM_B,
@@ -602,7 +602,7 @@ def run_ours(a):
     roof.update({
         "traffic": traffic,
         "traffic_note": "DRAM bytes per matvec of the kernel: ncu per-unit figures of this "
-                        "command, scaled by the units of one matvec",
+                        "matvec, scaled by the units of one matvec",
         "launches_per_step": kernels[dom]["launches"] / max(prof["mults"], 1) * batch,
         "ms_per_matvec": per_mult_ms,
         "ms_note": "per-kernel times come from a pass with CUDA events around every launch "
