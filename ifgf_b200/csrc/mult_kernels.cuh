@@ -286,7 +286,7 @@ struct UpArgs
 // Should a tabulated element be inactive in this child (the table works in
 // coordinates relative to the parent, the activation in absolute ones), the
 // node is recomputed from absolute coordinates as the reference does.
-template <int KIND, int N0, int N1, int N2>
+template <int KIND>
 __device__ __forceinline__ bool upward_fallback64(const UpArgs& a, int box, int el, int n, int cb,
                                                   const int* fm, cplx<double>& v_out)
 {
@@ -309,7 +309,7 @@ __device__ __forceinline__ bool upward_fallback64(const UpArgs& a, int box, int 
         return false;
     }
     to_local(fe, s, C.dmin, C.hf, C.hfi, C.nf, loc);
-    const cplx<double> v = Cheb<N0, N1, N2>::eval(a.fcoef + (size_t)gf * a.P_lo, loc, a.lo);
+    const cplx<double> v = Cheb<0, 0, 0>::eval(a.fcoef + (size_t)gf * a.P_lo, loc, a.lo);
     const double e0 = y[0] - xc[0], e1 = y[1] - xc[1], e2 = y[2] - xc[2];
     v_out = cmul(v, P::transfer(p0 * p0 + p1 * p1 + p2 * p2, e0 * e0 + e1 * e1 + e2 * e2, a.kp));
     return true;
@@ -1380,8 +1380,9 @@ constexpr size_t UP_STAGED_SMEM_MAX = 96 * 1024;
 // level's geometry table in groups of R sharing one child cone: one
 // coefficient gather serves R nodes.  Each node is updated once per child,
 // so the per-node sums in shared memory need no atomics.
-template <int KIND, int N0, int N1, int N2>
-__global__ void __launch_bounds__(UP_THREADS) upward_kernel(UpArgs a)
+// Runtime orders: the fixed ones stage the coefficient blocks (upward_staged64.cuh),
+// unless a row's run list leaves no room in shared memory.
+template <int KIND> __global__ void __launch_bounds__(UP_THREADS) upward_kernel(UpArgs a)
 {
     constexpr int R = 2;
     extern __shared__ double2 acc64[];
@@ -1419,7 +1420,7 @@ __global__ void __launch_bounds__(UP_THREADS) upward_kernel(UpArgs a)
                 {
                     cplx<double> v;
                     if (e[r].node >= 0 &&
-                        upward_fallback64<KIND, N0, N1, N2>(a, box, el, e[r].node, cb, fm, v))
+                        upward_fallback64<KIND>(a, box, el, e[r].node, cb, fm, v))
                     {
                         acc64[e[r].node].x += v.re;
                         acc64[e[r].node].y += v.im;
@@ -1432,7 +1433,7 @@ __global__ void __launch_bounds__(UP_THREADS) upward_kernel(UpArgs a)
             for (int r = 0; r < R; r++)
                 for (int d = 0; d < 3; d++)
                     x[r][d] = e[r].loc[d];
-            ChebMulti<double, N0, N1, N2, R>::eval(a.fcoef + (size_t)gf * a.P_lo, x, a.lo, vr, vi);
+            ChebMulti<double, 0, 0, 0, R>::eval(a.fcoef + (size_t)gf * a.P_lo, x, a.lo, vr, vi);
 #pragma unroll
             for (int r = 0; r < R; r++)
                 if (e[r].node >= 0)
@@ -2305,7 +2306,7 @@ static int run_mult(const MultPtrs& m, const void* d_w, void* d_u, bool real, cu
                 upward_mixed_kernel<KIND, N0, N1, N2>
                     <<<LL.n_up, UP_THREADS, m.P_hi * sizeof(float2), st>>>(ua);
             else
-                upward_kernel<KIND, 0, 0, 0>
+                upward_kernel<KIND>
                     <<<LL.n_up, UP_THREADS, m.P_hi * sizeof(double2), st>>>(ua);
             IFGF_CHECK_LAUNCH();
             if (hk)

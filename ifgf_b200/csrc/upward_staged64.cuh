@@ -79,7 +79,7 @@ template <int KIND>
 __device__ __noinline__ bool ups64_fallback(const UpArgs& a, int box, int el, int n, int cb,
                                             const int* fm, cplx<double>& v)
 {
-    return upward_fallback64<KIND, 0, 0, 0>(a, box, el, n, cb, fm, v);
+    return upward_fallback64<KIND>(a, box, el, n, cb, fm, v);
 }
 
 // Threads: blocks of more than 200 coefficients leave room for fewer CTAs per
