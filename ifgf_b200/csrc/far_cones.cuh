@@ -91,9 +91,9 @@ constexpr int FAR_CONE_THREADS = 128;
 // One warp per 32 consecutive places of the plan, four tiles of eight: lane =
 // place for the local coordinates and the centred factor, row lane / 4 of the
 // products for the sums; both views meet in the warp's shared memory.
-// At N = 1e6, p = 9 (3.9e8 pairs) the far field of a matvec takes 17.3 ms with
+// At N = 1e6, p = 9 (3.8e8 pairs) the far field of a matvec takes 17.0 ms with
 // the gather; the kernel that looks up every pair and reads its coefficients
-// lane by lane took 43.3.  At N = 2e5, p = 8 1.7 and 3.45 ms, N = 2e4 Laplace
+// lane by lane took 43.3.  At N = 2e5, p = 8 1.6 and 3.45 ms, N = 2e4 Laplace
 // 0.13 and 0.72, 4000 points 0.031 and 0.135.  The FP64 and
 // matrix pipes together are about 57 % busy at p = 8, issue slots 65 %.  A
 // first form gave a warp up to 64 places of one cone: its second batch of 32

@@ -132,10 +132,10 @@ __device__ __forceinline__ void node_position(const LevelGeom& G, int el, int n,
 
 // One CTA per coarse cone of a leaf box (blockIdx.y: chunk of its nodes): sum
 // over the leaf's sources, staged in shared memory, at NPT nodes per thread
-// that share each source's loads.  Bound by the FP64 pipe (about 42 of its
+// that share each source's loads.  Bound by the FP64 pipe (about 44 of its
 // instructions per evaluation, issued at three quarters of the 57 FMAs per
 // clock and SM that a loop of independent FMAs reaches): at N = 1e6, p = 9
-// 27.0 ms per matvec with the library functions, 17.9 with the forms of
+// 27.0 ms per matvec with the library functions, 18.0 with the forms of
 // device_math.cuh.  Three CTAs of 256 threads per SM (80 registers): two ran
 // 20.2 ms; one node per thread 21.1, four at 182 registers 20.1.
 template <int KIND>

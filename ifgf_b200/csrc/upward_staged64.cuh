@@ -127,7 +127,7 @@ constexpr int UPS64_R = 2;
 // the few blocks a warp reads and feeds 2 R FMAs) and the latency of the
 // chunks' copies.  The kernel it replaces gathered every coefficient from
 // global memory: at N = 1e6, p = 9 the transfer took 57.4 ms per matvec and
-// takes 27.7; at N = 2e5, p = 8 4.1 and 2.5.  Measured at N = 1e6 for entries
+// takes 28.0; at N = 2e5, p = 8 4.1 and 2.5.  Measured at N = 1e6 for entries
 // per thread / threads / KB of blocks / CTAs per SM: 2 / 64 / 16 / 8 28.3 ms,
 // 2 / 64 / 16 / 10 29.7, 2 / 96 / 24 / 6 32.9, 4 / 64 / 24 / 6 30.1,
 // 4 / 64 / 16 / 4 35.6, 4 / 32 / 8 / 12 35.5: warps in flight are worth more

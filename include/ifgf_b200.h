@@ -112,8 +112,12 @@ int ifgf_set_upward_path(ifgf_operator* op, int path);
  * keep plans of their own, one per precision used (pairs sorted by cone, a
  * value array; about 25 bytes per pair in FP64, 17 mixed: 9.8 and 6.7 GB at
  * that size, "far_cones" in the stats), built on the first call outside a
- * stream capture where it takes at most a quarter of the free device memory;
- * without it the far kernel looks the cones up (same results to rounding).
+ * stream capture (which then waits for its stream) where it takes at most a
+ * quarter of the free device memory; without it the far kernel looks the
+ * cones up (same results to rounding).  Another allocation of the library
+ * that fails frees these plans, of every operator on the device, except those
+ * a capture has recorded; a plan that found no memory or was freed so is
+ * tried again every 16 matvecs ("refused" in the stats meanwhile).
  * enable = 0 frees them too, unless a capture has recorded one (then the next
  * init does).  No reference counterpart. */
 int ifgf_set_far_plan(ifgf_operator* op, int enable);
