@@ -319,7 +319,7 @@ void build_far_cones(const FarConeBuild& b, FarConePlan& plan)
 // far boxes si, si + S, ... (S = threads / targets); the S sums and the near
 // sum are added in a fixed order and written in the caller's order.  Bound
 // by memory (20 bytes a pair, mixed 12); with one value in flight per thread
-// instead of eight the FP64 far field at N = 1e6 took 17.9 ms instead of 17.3.
+// the FP64 far field at N = 1e6 took 17.9 ms, with eight 17.3.
 template <typename V>
 __global__ void __launch_bounds__(THREADS)
     far_gather_kernel(FarConePtrs fc, const int* __restrict__ tl_first,

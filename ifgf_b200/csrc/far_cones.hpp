@@ -56,7 +56,8 @@ constexpr int FAR_CONES_RETRY = 16;
 
 // Fills `plan`, or leaves it empty: with `refused` set for no far pairs or 2^31
 // places or more, with `wait` set where it would take more than a quarter of
-// the free device memory or finds none (3.9e8 pairs take 12 ms).  Runs on the build's stream and waits for that one alone.
+// the free device memory or finds none (3.9e8 pairs take 12 ms).  Runs on the
+// build's stream and waits for that one alone.
 void build_far_cones(const FarConeBuild& b, FarConePlan& plan);
 
 } // namespace ifgf
